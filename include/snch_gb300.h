@@ -264,8 +264,13 @@ int snch_set_traversal(snch_scene_t scene, int mode);
 /*   SNCH_OPT_PACKET           warp packets for the binary near-first nearest and
  *                             silhouette searches: a warp's 32 queries walk one shared
  *                             traversal, each lane applying its own tests and keeping its
- *                             own answer. 2 (default): for Morton-ordered batches (nearest
- *                             batches also need at least 1 query per triangle); 1:
+ *                             own answer. 2 (default): the library chooses by size: small
+ *                             batches (unordered, or up to 98,304 nearest / 131,072
+ *                             silhouette queries) run one query per warp, its 32 lanes
+ *                             expanding 32 nodes of that query's search at a time;
+ *                             larger ordered batches run as packets (nearest
+ *                             batches also need at least 1 query per triangle), whose
+ *                             last, long packets finish one query per warp. 1: packets
  *                             always; 0: never (each lane walks its own). Same distances;
  *                             the silhouette edge id / nearest index equals the per-lane
  *                             one except on an exact distance tie that falls on a
@@ -281,8 +286,10 @@ int snch_set_traversal(snch_scene_t scene, int mode);
  *                             refilled with 32 consecutive packets at a time (same
  *                             packets, same answers); ray batches of at least 4 times
  *                             this run the same way, 32 rays (one per lane) per take.
- *                             Default 2^19 (measured: silhouette packets faster from
- *                             524,288 queries, rays from about 2M); >= 1. */
+ *                             Default 2^19, >= 1. Where SNCH_OPT_PACKET is left at 2,
+ *                             packets of smaller batches run persistent too. Batches
+ *                             below 2^20 queries draw packets from the batch's counter
+ *                             instead of the pools. */
 #define SNCH_OPT_PACKET_PERSISTENT_MIN 19
 /*   SNCH_OPT_OUTPUT_SCATTER   1: the results of a Morton-ordered, unseeded batch are
  *                             written in batch order to a temporary and then moved to

@@ -835,12 +835,12 @@ SNCH_DEV void leaf_silhouette_fast(const TreeView &t, uint32_t pos, f3 o, bool f
     }
 }
 
-// owned edge k of the leaf at sorted position pos (rank: the leaf's rank) as a
-// silhouette candidate
-SNCH_DEV void edge_candidate(const TreeView &t, uint32_t pos, uint32_t k, uint32_t rank, f3 o, bool flip, float &best,
-                             uint32_t &best_key, int32_t &best_edge)
+// the edge record at slot (3 x sorted leaf position + edge number) with tie key
+// rank * 4 + edge number, as a silhouette candidate
+SNCH_DEV void edge_record_candidate(const TreeView &t, uint64_t slot, uint32_t key, f3 o, bool flip, float &best,
+                                    uint32_t &best_key, int32_t &best_edge)
 {
-    const float4 *e = reinterpret_cast<const float4 *>(t.edges + 3 * (uint64_t)pos + k);
+    const float4 *e = reinterpret_cast<const float4 *>(t.edges + slot);
     const float4 ea = __ldg(e), eb = __ldg(e + 1);
     const f3 pa = mk(ea.x, ea.y, ea.z), pb = mk(eb.x, eb.y, eb.z);
     f3 cp;
@@ -860,13 +860,19 @@ SNCH_DEV void edge_candidate(const TreeView &t, uint32_t pos, uint32_t k, uint32
     }
     if (!is_sil)
         return;
-    const uint32_t key = rank * 4u + k;
     if (d < best || best_edge < 0 || (d > 0.0f ? key > best_key : key < best_key))
     {
         best = d;
         best_key = key;
         best_edge = __float_as_int(eb.w);
     }
+}
+
+// owned edge k of the leaf at sorted position pos (rank: the leaf's rank)
+SNCH_DEV void edge_candidate(const TreeView &t, uint32_t pos, uint32_t k, uint32_t rank, f3 o, bool flip, float &best,
+                             uint32_t &best_key, int32_t &best_edge)
+{
+    edge_record_candidate(t, 3 * (uint64_t)pos + k, rank * 4u + k, o, flip, best, best_key, best_edge);
 }
 
 // the same for a leaf reached through its parent: rank and owned-edge count
@@ -1476,13 +1482,19 @@ constexpr uint32_t kPoolSlots = 1024;                  // pools (SM id modulo kP
 constexpr uint64_t kPoolChunk = SNCH_POOL_CHUNK;  // packets per refill
 constexpr unsigned long long kPoolDone = (1ull << 40) - 1ull;
 constexpr uint32_t kPoolSpins = 1u << 16;
+// Smaller batches take every packet straight from the counter: a chunk of
+// neighbouring packets is neighbouring work, and where a batch is only a few chunks
+// per SM, one SM's chunk is the expensive region (silhouettes, pools / counter, ms:
+// 1,280-triangle sphere, 140k queries 0.86 / 0.50; 20,480 triangles, 1M 14.9 / 14.3;
+// 2M-triangle scene, 1M 5.56 / 5.28, 4M 11.8 / 12.0).
+constexpr unsigned long long kPoolMinPackets = 1ull << 15;
 // work[0]: the batch-wide packet counter, work[1 + s]: pool s (zeroed before
 // the launch). Returns a packet index (>= total_packets: the unused end of the
 // last chunk, take again; at most kPoolChunk of those before the pool is done)
 // or ~0 when every packet has been handed out.
 __device__ __noinline__ unsigned long long take_packet(unsigned long long *work, unsigned long long total_packets)
 {
-    if (!kPacketPools)
+    if (!kPacketPools || total_packets < kPoolMinPackets)
     {
         const unsigned long long p = atomicAdd(work, 1ull);
         return p < total_packets ? p : ~0ull;
@@ -1512,6 +1524,61 @@ __device__ __noinline__ unsigned long long take_packet(unsigned long long *work,
     return p < total_packets ? p : ~0ull;
 }
 
+// Long packets at the end of a batch. The last packets of a batch decide when it
+// ends, and a packet deep inside a closed mesh expands thousands of nodes, one
+// after the other, while the SMs around it have run dry. So a packet that has
+// popped kDeferPops entries and finds the batch handed out stops, and the queries
+// it still searches for go to a list with the candidate each has; the launch
+// that follows finishes them one query per warp (coop.cuh), from the root and
+// bounded by that candidate. The answer is the minimum over the leaves reached
+// either way, ties by rank, so it does not depend on where a search stopped.
+// Measured, without / with (ms): 1M nearest queries around a 20,480-triangle sphere
+// 3.32 / 1.44, 200k silhouette queries there 7.8 / 4.0, 2.4M silhouette queries of 24
+// meshes (one closed, 81,920 triangles) 91 / 36. On 16M-query batches of the
+// 2M-triangle scene, whose packets are all short, the pop count costs more than the
+// end of the batch gains (nearest 10.75 / 10.96, silhouette 33.97 / 34.47); checking
+// every step instead of every pop cost 12 % there, and leaving after 64 pops instead
+// of 128 sent packets to the list that were about to end (nearest 11.23).
+constexpr int kDeferPops = 128;  // the batch's counter is read every so many pops
+struct DeferArgs
+{
+    uint4 *list = nullptr;      // (query, candidate's distance bits, rank or key, triangle or edge); nullptr: off
+    uint32_t *count = nullptr;  // entries reserved; may pass capacity, by entries that are not in the list
+    uint32_t capacity = 0;
+};
+// Whether the packet stops here: the lanes whose queries went to the list, 0 = it
+// goes on (the batch is not handed out yet, or the list is full). work: the
+// batch-wide packet counter, total: the batch's queries, lanes: those not yet
+// started. Called by all lanes of the warp.
+__device__ __noinline__ uint32_t leave_packet(DeferArgs d, const unsigned long long *work, unsigned long long total,
+                                              const uint32_t *st_mask, int sp, uint32_t lanes, uint32_t q,
+                                              float best, uint32_t rank, uint32_t id)
+{
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    if (!d.list)
+        return 0u;
+    unsigned long long v = 0;
+    if (lane == 0)
+        asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(work) : "memory");
+    if (32ull * __shfl_sync(full, v, 0) < total)
+        return 0u;
+    // the lanes with work on the stack
+    uint32_t left = (lane < sp ? st_mask[lane] : 0u) | (lane + 32 < sp ? st_mask[lane + 32] : 0u);
+    left = __reduce_or_sync(full, left) | lanes;
+    const uint32_t cnt = (uint32_t)__popc(left);
+    uint32_t base = 0;
+    if (lane == 0)
+        base = atomicAdd(d.count, cnt);
+    base = __shfl_sync(full, base, 0);
+    const bool fits = (uint64_t)base + cnt <= d.capacity;
+    const uint64_t at = (uint64_t)base + __popc(left & ((1u << lane) - 1u));
+    if (((left >> lane) & 1u) && at < d.capacity)  // places that are reserved but not used: kInvalid
+        d.list[at] = make_uint4(fits ? q : kInvalid, __float_as_uint(best), rank, id);
+    return fits ? left : 0u;
+}
+static_assert(kStackDepth <= 64, "leave_packet reads two stack entries a lane");
+
 // per-lane start of a packet: lanes of a batched query set may search
 // different meshes; the warp runs one packet per distinct root
 struct PacketLane
@@ -1533,15 +1600,16 @@ SNCH_DEV uint32_t child_slot(uint32_t slot, uint32_t k, uint32_t top_slots)
     return slot < top_slots && c < top_slots ? c : kNoSlot;
 }
 
-template <bool kStats, bool kTop = false>
+template <bool kStats, bool kTop = false, bool kDefer = false>
 SNCH_DEV void nearest_packet_chunk(const TreeView &t, const float *__restrict__ pts, int64_t n,
                                    uint32_t *__restrict__ out_idx, float *__restrict__ out_dist,
                                    uint32_t *__restrict__ stats, const SeedArgs &seed, int64_t qi, uint32_t *st_node,
                                    uint32_t *st_mask, uint8_t *st_slot = nullptr, const InnerRec *s_top = nullptr,
-                                   uint32_t top_slots = 0)
+                                   uint32_t top_slots = 0, const DeferArgs &defer = DeferArgs(),
+                                   const unsigned long long *work = nullptr)
 {
     const int lane = threadIdx.x & 31;
-    const bool valid = qi < query_count(t, n);
+    bool valid = qi < query_count(t, n);
     if (__ballot_sync(0xffffffffu, valid) == 0u)
         return;
     const int64_t q = valid ? query_index(t, qi) : 0;
@@ -1558,6 +1626,7 @@ SNCH_DEV void nearest_packet_chunk(const TreeView &t, const float *__restrict__ 
     if (valid && qr.node != kInvalid && qr.node >= ni)  // a one-triangle tree or mesh
         leaf_nearest_fast(t, qr.node - ni, p, best, best_rank, nearest);
     bool overflow = false;
+    int pops = kDeferPops;
     uint32_t pending = __ballot_sync(0xffffffffu, valid && qr.node != kInvalid && qr.node < ni);
     while (pending)
     {
@@ -1578,6 +1647,18 @@ SNCH_DEV void nearest_packet_chunk(const TreeView &t, const float *__restrict__ 
             {
                 if (sp == 0)
                     break;
+                if (kDefer && --pops == 0)
+                {
+                    pops = kDeferPops;
+                    const uint32_t left = leave_packet(defer, work, (unsigned long long)query_count(t, n), st_mask, sp,
+                                                       pending, (uint32_t)q, best, best_rank, nearest);
+                    if (left)
+                    {
+                        valid = valid && !((left >> lane) & 1u);
+                        pending = 0u;
+                        break;
+                    }
+                }
                 --sp;
                 node = st_node[sp];
                 mask = st_mask[sp];
@@ -1764,10 +1845,11 @@ inline size_t top_smem_bytes(uint32_t slots, bool cones)
 #ifndef SNCH_NEAR_PACKET_MIN_BLOCKS
 #define SNCH_NEAR_PACKET_MIN_BLOCKS 7
 #endif
-template <bool kTop>
+template <bool kTop, bool kDefer = !kTop>
 __global__ void __launch_bounds__(128, SNCH_NEAR_PACKET_MIN_BLOCKS)
     nearest_packet_persistent_kernel(TreeView t, const float *__restrict__ pts, int64_t n, uint32_t *__restrict__ out_idx,
-                                     float *__restrict__ out_dist, SeedArgs seed, unsigned long long *counter)
+                                     float *__restrict__ out_dist, SeedArgs seed, DeferArgs defer,
+                                     unsigned long long *counter)
 {
     __shared__ uint32_t st_node[kPacketWarps][kStackDepth];
     __shared__ uint32_t st_mask[kPacketWarps][kStackDepth];
@@ -1799,23 +1881,24 @@ __global__ void __launch_bounds__(128, SNCH_NEAR_PACKET_MIN_BLOCKS)
         }
         empty_takes = 0;
         const unsigned long long base = packet * 32ull;
-        nearest_packet_chunk<false, kTop>(t, pts, n, out_idx, out_dist, nullptr, seed, (int64_t)base + lane,
-                                          st_node[w], st_mask[w], st_slot[w], s_top, top_slots);
+        nearest_packet_chunk<false, kTop, kDefer>(t, pts, n, out_idx, out_dist, nullptr, seed, (int64_t)base + lane,
+                                          st_node[w], st_mask[w], st_slot[w], s_top, top_slots, defer, counter);
         __syncwarp();
     }
 }
 
 // one warp's packet: the 32 queries qi .. qi + 31 (lane order) of the batch
-template <bool kStats, bool kTop = false>
+template <bool kStats, bool kTop = false, bool kDefer = false>
 SNCH_DEV void silhouette_packet_chunk(const TreeView &t, const float *__restrict__ pts, const uint8_t *__restrict__ flips,
                                       int64_t n, float *__restrict__ out_dist, int32_t *__restrict__ out_edge,
                                       uint32_t *__restrict__ stats, const SeedArgs &seed, int64_t qi,
                                       uint32_t *st_node, uint32_t *st_mask, uint8_t *st_slot = nullptr,
                                       const InnerRec *s_top = nullptr, const InnerConeRec *s_topc = nullptr,
-                                      uint32_t top_slots = 0)
+                                      uint32_t top_slots = 0, const DeferArgs &defer = DeferArgs(),
+                                   const unsigned long long *work = nullptr)
 {
     const int lane = threadIdx.x & 31;
-    const bool valid = qi < query_count(t, n);
+    bool valid = qi < query_count(t, n);
     if (__ballot_sync(0xffffffffu, valid) == 0u)
         return;
     const int64_t q = valid ? query_index(t, qi) : 0;
@@ -1830,6 +1913,7 @@ SNCH_DEV void silhouette_packet_chunk(const TreeView &t, const float *__restrict
     if (valid && qr.node != kInvalid && qr.node >= ni)  // a one-triangle tree or mesh
         leaf_silhouette_fast(t, qr.node - ni, p, flip, best, best_key, best_edge, n_edge);
     bool overflow = false;
+    int pops = kDeferPops;
     uint32_t pending = __ballot_sync(0xffffffffu, valid && qr.node != kInvalid && qr.node < ni);
     while (pending)
     {
@@ -1850,6 +1934,18 @@ SNCH_DEV void silhouette_packet_chunk(const TreeView &t, const float *__restrict
             {
                 if (sp == 0)
                     break;
+                if (kDefer && --pops == 0)
+                {
+                    pops = kDeferPops;
+                    const uint32_t left = leave_packet(defer, work, (unsigned long long)query_count(t, n), st_mask, sp,
+                                                       pending, (uint32_t)q, best, best_key, (uint32_t)best_edge);
+                    if (left)
+                    {
+                        valid = valid && !((left >> lane) & 1u);
+                        pending = 0u;
+                        break;
+                    }
+                }
                 --sp;
                 node = st_node[sp];
                 mask = st_mask[sp];
@@ -1990,11 +2086,11 @@ __global__ void __launch_bounds__(128, SNCH_SIL_PACKET_MIN_BLOCKS)
 }
 
 // the same packets, persistent (see nearest_packet_persistent_kernel)
-template <bool kTop>
+template <bool kTop, bool kDefer = !kTop>
 __global__ void __launch_bounds__(128, SNCH_SIL_PACKET_MIN_BLOCKS)
     silhouette_packet_persistent_kernel(TreeView t, const float *__restrict__ pts, const uint8_t *__restrict__ flips,
                                         int64_t n, float *__restrict__ out_dist, int32_t *__restrict__ out_edge,
-                                        SeedArgs seed, unsigned long long *counter)
+                                        SeedArgs seed, DeferArgs defer, unsigned long long *counter)
 {
     __shared__ uint32_t st_node[kPacketWarps][kStackDepth];
     __shared__ uint32_t st_mask[kPacketWarps][kStackDepth];
@@ -2027,11 +2123,13 @@ __global__ void __launch_bounds__(128, SNCH_SIL_PACKET_MIN_BLOCKS)
         }
         empty_takes = 0;
         const unsigned long long base = packet * 32ull;
-        silhouette_packet_chunk<false, kTop>(t, pts, flips, n, out_dist, out_edge, nullptr, seed, (int64_t)base + lane,
-                                             st_node[w], st_mask[w], st_slot[w], s_top, s_topc, top_slots);
+        silhouette_packet_chunk<false, kTop, kDefer>(t, pts, flips, n, out_dist, out_edge, nullptr, seed, (int64_t)base + lane,
+                                             st_node[w], st_mask[w], st_slot[w], s_top, s_topc, top_slots, defer, counter);
         __syncwarp();
     }
 }
+
+#include "coop.cuh"
 
 // ------------------------------------------------------------------ persistent forms
 // The per-query traversals above run one query per thread; a warp then runs
@@ -3160,6 +3258,22 @@ inline bool packet_dense(const TreeView &t, int packet, int64_t n)
 {
     return packet == 1 || (uint64_t)n >= kPacketNearestMinQueriesPerTri * t.num_tris;
 }
+// Small batches run one query per warp (coop.cuh) when the search form is left to
+// the library: automatic packets, binary records, the default block. Measured, one
+// query per lane / per warp (ms), 2M-triangle scene: nearest 4,096 queries 0.26 /
+// 0.05, 20,000 0.30 / 0.16, 64,000 0.43 / 0.44; silhouette 1.07 / 0.13, 1.78 / 0.38,
+// 1.89 / 0.93; 20,480-triangle sphere: nearest 0.93 / 0.09, 1.27 / 0.20, 1.30 / 0.42;
+// silhouette 9.9 / 0.43, 11.2 / 0.84, 12.1 / 2.0. Ordered batches: packets (with their
+// second launch) win from about 100k nearest and 130k silhouette queries (131k:
+// sphere 0.72 against 0.88, 3.3 / 3.5; 1,280 triangles 1.02 / 0.93); nearest batches
+// with fewer than one query per 4 triangles stay one per lane (100k, 2M triangles:
+// 0.50 / 0.69).
+inline bool coop_ok(const TreeView &t, int packet, int width, int block, bool persistent, const SeedArgs &seed)
+{
+    return t.near_first && packet == 2 && width == 2 && block == 128 && !persistent && !seed.cap && t.num_tris > 1 &&
+           !t.order_count && !t.out_batch_order_enabled;
+}
+constexpr int64_t kCoopNearestMax = 98304, kCoopSilhouetteMax = 131072;
 // the wide searches serve near-first, one-thread-per-query, uncapped launches
 // over a tree whose wide records of that width exist
 inline bool wide_ok(const TreeView &t, int width, bool persistent, const SeedArgs &seed)
@@ -3169,10 +3283,9 @@ inline bool wide_ok(const TreeView &t, int width, bool persistent, const SeedArg
     return (width == 4 && t.wide4 && t.wide4_of) || (width == 8 && t.wide8 && t.wide8_of);
 }
 // persistent launch: as many 128-thread blocks as the GPU holds at once (fewer for
-// small batches), and a zeroed 64-bit work counter of its own (stream-ordered
-// allocation, so concurrent calls on other streams do not share it)
-template <typename... KArgs, typename... Args>
-cudaError_t launch_persistent_smem(void (*kernel)(KArgs...), size_t smem, int64_t n, cudaStream_t st, Args... args)
+// small batches)
+template <typename... KArgs>
+cudaError_t persistent_grid(void (*kernel)(KArgs...), size_t smem, int64_t n, unsigned &grid, unsigned &num_sms)
 {
     int dev = 0, sms = 0, per_sm = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -3180,16 +3293,26 @@ cudaError_t launch_persistent_smem(void (*kernel)(KArgs...), size_t smem, int64_
         e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e == cudaSuccess)
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 128, smem);
+    const int64_t need = (n + 127) / 128;
+    grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(need, (int64_t)sms * std::max(per_sm, 1)));
+    num_sms = (unsigned)sms;
+    return e;
+}
+// the work counter and, for the packet searches, the per-SM packet pools
+constexpr size_t kWorkBytes = (1 + kPoolSlots) * sizeof(unsigned long long);
+// with a zeroed 64-bit work counter of its own (stream-ordered allocation, so
+// concurrent calls on other streams do not share it)
+template <typename... KArgs, typename... Args>
+cudaError_t launch_persistent_smem(void (*kernel)(KArgs...), size_t smem, int64_t n, cudaStream_t st, Args... args)
+{
+    unsigned grid = 0, sms = 0;
+    cudaError_t e = persistent_grid(kernel, smem, n, grid, sms);
     if (e != cudaSuccess)
         return e;
-    const int64_t need = (n + 127) / 128;
-    const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(need, (int64_t)sms * std::max(per_sm, 1)));
     unsigned long long *counter = nullptr;
-    // the work counter and, for the packet searches, the per-SM packet pools
-    constexpr size_t work_bytes = (1 + kPoolSlots) * sizeof(unsigned long long);
-    if ((e = scratch_alloc_raw(reinterpret_cast<void **>(&counter), work_bytes, st)) != cudaSuccess)
+    if ((e = scratch_alloc_raw(reinterpret_cast<void **>(&counter), kWorkBytes, st)) != cudaSuccess)
         return e;
-    e = cudaMemsetAsync(counter, 0, work_bytes, st);
+    e = cudaMemsetAsync(counter, 0, kWorkBytes, st);
     if (e == cudaSuccess)
     {
         kernel<<<grid, 128, smem, st>>>(args..., counter);
@@ -3203,6 +3326,42 @@ template <typename... KArgs, typename... Args>
 cudaError_t launch_persistent(void (*kernel)(KArgs...), int64_t n, cudaStream_t st, Args... args)
 {
     return launch_persistent_smem(kernel, 0, n, st, args...);
+}
+// Persistent packets whose long ones end in a second launch (DeferArgs): kernel
+// takes (args..., defer, counter), finish(list, words, sms) launches the rest. The
+// list holds what can be in flight once the batch is handed out: a packet per
+// warp and a chunk per SM's pool.
+template <typename Finish, typename... KArgs, typename... Args>
+cudaError_t launch_deferring(void (*kernel)(KArgs...), int64_t n, cudaStream_t st, Finish finish, Args... args)
+{
+    unsigned grid = 0, sms = 0;
+    cudaError_t e = persistent_grid(kernel, 0, n, grid, sms);
+    if (e != cudaSuccess)
+        return e;
+    const int64_t in_flight = 32 * (4 * (int64_t)grid + (int64_t)kPoolChunk * sms);
+    DeferArgs d;
+    d.capacity = (uint32_t)std::min<int64_t>((n + 31) / 32 * 32, in_flight);
+    constexpr size_t head = (kWorkBytes + 8 + 255) / 256 * 256;  // counter, pools, list count, list position
+    char *scratch = nullptr;
+    if ((e = scratch_alloc_raw(reinterpret_cast<void **>(&scratch), head + 16 * (size_t)d.capacity, st)) != cudaSuccess)
+        return e;
+    d.count = reinterpret_cast<uint32_t *>(scratch + kWorkBytes);
+    d.list = reinterpret_cast<uint4 *>(scratch + head);
+    e = cudaMemsetAsync(scratch, 0, head, st);
+    if (e == cudaSuccess)
+    {
+        kernel<<<grid, 128, 0, st>>>(args..., d, reinterpret_cast<unsigned long long *>(scratch));
+        note_launch();
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess)
+    {
+        finish(d, 16 * sms);
+        note_launch();
+        e = cudaGetLastError();
+    }
+    const cudaError_t f = cudaFreeAsync(scratch, st);
+    return e != cudaSuccess ? e : f;
 }
 // Results of an unseeded, fully Morton-ordered batch are written at their batch
 // position into a stream-ordered temporary (warp-contiguous, coalesced stores)
@@ -3287,7 +3446,10 @@ cudaError_t launch_nearest(const TreeView &t0, const float *pts, int64_t n, uint
         return cudaSuccess;
     TreeView t = t0;
     const bool persistent = (t.persistent & 1) != 0;
-    const bool packets = packet_ok(t, t.packet_near, t.width_near, seed) && packet_dense(t, t.packet_near, n);
+    const bool dense = packet_dense(t, t.packet_near, n);
+    const bool coop = !stats && n <= kCoopNearestMax && (!t.order || 4 * (uint64_t)n >= t.num_tris) &&
+                      coop_ok(t, t.packet_near, t.width_near, t.block_near, persistent, seed);
+    const bool packets = !coop && dense && packet_ok(t, t.packet_near, t.width_near, seed);
     const bool wide = !packets && wide_ok(t, t.width_near, persistent, seed);
     const bool lane_persistent = !packets && !wide && !stats && t.near_first && t.num_tris > 1 && persistent;
     // the kernels below that write at out_pos() (all but the lane-refill and reference-order ones)
@@ -3313,12 +3475,26 @@ cudaError_t launch_nearest(const TreeView &t0, const float *pts, int64_t n, uint
         // 6 % slower on 1M-query batches. The counters' pass keeps the grid form.
         if (stats)
             nearest_packet_kernel<true><<<grid_for(n, 128), 128, 0, st>>>(t, pts, n, idx, dist, stats, seed);
-        else if (n >= t.packet_persistent_min)
+        else if (t.top_slots && !t.query_mesh && n >= t.packet_persistent_min)
         {
-            e = t.top_slots && !t.query_mesh
-                    ? launch_persistent_smem(nearest_packet_persistent_kernel<true>, top_smem_bytes(t.top_slots, false),
-                                             n, st, t, pts, n, idx, dist, seed)
-                    : launch_persistent(nearest_packet_persistent_kernel<false>, n, st, t, pts, n, idx, dist, seed);
+            e = launch_persistent_smem(nearest_packet_persistent_kernel<true>, top_smem_bytes(t.top_slots, false), n,
+                                       st, t, pts, n, idx, dist, seed, DeferArgs());
+            launched = true;
+        }
+        else if (n >= t.packet_persistent_min || t.packet_near == 2)
+        {
+            // with a second launch for the batch's last, long packets; not where results
+            // are written in batch order (its list has 32-bit queries only)
+            if (t.out_batch_order || n >= INT64_C(0xFFFFFFFF))
+                e = launch_persistent(nearest_packet_persistent_kernel<false, false>, n, st, t, pts, n, idx, dist, seed,
+                                      DeferArgs());
+            else
+                e = launch_deferring(
+                    nearest_packet_persistent_kernel<false>, n, st,
+                    [&](const DeferArgs &d, unsigned blocks) {
+                        nearest_finish_kernel<<<blocks, 32 * kCoopWarps, 0, st>>>(t, pts, idx, dist, seed, d);
+                    },
+                    t, pts, n, idx, dist, seed);
             launched = true;
         }
         else
@@ -3342,6 +3518,8 @@ cudaError_t launch_nearest(const TreeView &t0, const float *pts, int64_t n, uint
                         : launch_persistent(nearest_persistent_kernel<false>, n, st, t, pts, n, idx, dist, seed);
         launched = true;
     }
+    else if (coop)
+        nearest_coop_kernel<<<grid_for(n, kCoopWarps), 32 * kCoopWarps, 0, st>>>(t, pts, n, idx, dist, seed);
     else if (t.near_first && t.block_near == 64)
         nearest_fast_kernel<false, 64><<<grid_for(n, 64), 64, 0, st>>>(t, pts, n, idx, dist, nullptr, seed);
     else if (t.near_first && t.block_near == 256)
@@ -3372,7 +3550,9 @@ cudaError_t launch_silhouette(const TreeView &t0, const float *pts, const uint8_
         return cudaSuccess;
     TreeView t = t0;
     const bool persistent = (t.persistent & 2) != 0;
-    const bool packets = packet_ok(t, t.packet_sil, t.width_sil, seed);
+    const bool coop = !stats && n <= kCoopSilhouetteMax &&
+                      coop_ok(t, t.packet_sil, t.width_sil, t.block_sil, persistent, seed);
+    const bool packets = !coop && packet_ok(t, t.packet_sil, t.width_sil, seed);
     const bool wide = !packets && wide_ok(t, t.width_sil, persistent, seed);
     const bool lane_persistent = !packets && !wide && !stats && t.near_first && t.num_tris > 1 && persistent;
     const bool supports = packets || wide || (t.near_first && !lane_persistent);
@@ -3395,14 +3575,24 @@ cudaError_t launch_silhouette(const TreeView &t0, const float *pts, const uint8_
         if (stats)
             silhouette_packet_kernel<true>
                 <<<grid_for(n, 128), 128, 0, st>>>(t, pts, flip, n, dist, edge, stats, seed);
-        else if (n >= t.packet_persistent_min)
+        else if (t.top_slots && !t.query_mesh && n >= t.packet_persistent_min)
         {
-            e = t.top_slots && !t.query_mesh
-                    ? launch_persistent_smem(silhouette_packet_persistent_kernel<true>,
-                                             top_smem_bytes(t.top_slots, true), n, st, t, pts, flip, n, dist, edge,
-                                             seed)
-                    : launch_persistent(silhouette_packet_persistent_kernel<false>, n, st, t, pts, flip, n, dist, edge,
-                                        seed);
+            e = launch_persistent_smem(silhouette_packet_persistent_kernel<true>, top_smem_bytes(t.top_slots, true), n,
+                                       st, t, pts, flip, n, dist, edge, seed, DeferArgs());
+            launched = true;
+        }
+        else if (n >= t.packet_persistent_min || t.packet_sil == 2)
+        {
+            if (t.out_batch_order || n >= INT64_C(0xFFFFFFFF))
+                e = launch_persistent(silhouette_packet_persistent_kernel<false, false>, n, st, t, pts, flip, n, dist, edge,
+                                      seed, DeferArgs());
+            else
+                e = launch_deferring(
+                    silhouette_packet_persistent_kernel<false>, n, st,
+                    [&](const DeferArgs &d, unsigned blocks) {
+                        silhouette_finish_kernel<<<blocks, 32 * kCoopWarps, 0, st>>>(t, pts, flip, dist, edge, seed, d);
+                    },
+                    t, pts, flip, n, dist, edge, seed);
             launched = true;
         }
         else
@@ -3428,6 +3618,8 @@ cudaError_t launch_silhouette(const TreeView &t0, const float *pts, const uint8_
                 : launch_persistent(silhouette_persistent_kernel<false>, n, st, t, pts, flip, n, dist, edge, seed);
         launched = true;
     }
+    else if (coop)
+        silhouette_coop_kernel<<<grid_for(n, kCoopWarps), 32 * kCoopWarps, 0, st>>>(t, pts, flip, n, dist, edge, seed);
     else if (t.near_first && t.block_sil == 64)
         silhouette_fast_kernel<false, 64><<<grid_for(n, 64), 64, 0, st>>>(t, pts, flip, n, dist, edge, nullptr, seed);
     else if (t.near_first && t.block_sil == 256)

@@ -1,0 +1,98 @@
+"""Small batches run one query per warp, and the last long packets of a larger batch
+finish that way: the answers equal the one-query-per-lane searches bit for bit (the
+same minimum over the same leaves, ties by rank), at the edges of the size rules, on
+meshes from one triangle up, inside closed meshes, seeded, and in batched scenes."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def snch():
+    import torch
+    assert torch.cuda.is_available(), "GPU tests need a CUDA device"
+    import snch_lbvh_gb300
+    return snch_lbvh_gb300
+
+
+def mesh(level):
+    from snch_lbvh_gb300 import meshes
+    if level >= 0:
+        return meshes.noisy_icosphere(level, 1.0, 0.01, seed=level + 1)
+    v = np.array([[0, 0, 0], [1, 0, 0], [0, 1, 0], [1, 1, 0.5]], np.float32)
+    return v, np.array([[0, 1, 2], [1, 3, 2]], np.int32)[:-level]  # -1: one triangle, -2: two
+
+
+def scene(snch, level):
+    s = snch.Scene(*mesh(level))
+    s.compute_silhouettes()
+    s.build_bvh()
+    return s
+
+
+def points(n, seed=0):
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    return ((2 * torch.rand(n, 3, generator=g, device="cuda") - 1) * 1.2,
+            (torch.rand(n, generator=g, device="cuda") < 0.5).to(torch.uint8))
+
+
+def both_forms(snch, s, run):
+    """run() with one query per lane, then with the form left to the library."""
+    s.set_option(snch.OPT_PACKET, 0)
+    a = run()
+    s.set_option(snch.OPT_PACKET, 2)
+    b = run()
+    assert s.device_status() == 0
+    return a, b
+
+
+def same(a, b):
+    import torch
+    for x, y in zip(a, b):
+        assert torch.equal(x.view(torch.int32), y.view(torch.int32)), int((x != y).sum())
+
+
+@pytest.mark.parametrize("level", [-1, -2, 0, 2, 4])
+@pytest.mark.parametrize("n", [1, 2, 3, 31, 1000])
+def test_small_batches(snch, level, n):
+    s = scene(snch, level)
+    p, f = points(n, seed=n)
+    same(*both_forms(snch, s, lambda: s.query_nearest(p) + s.query_silhouette(p, f)))
+
+
+# around the sizes where a batch is ordered (65,536), where nearest (98,304) and
+# silhouette (131,072) batches become packets, and where packets draw from the
+# per-SM pools (2^15 packets), closed mesh: packets of thousands of steps
+@pytest.mark.parametrize("n", [65_535, 65_536, 98_304, 98_305, 131_072, 131_073, 32 * 2**15 - 31, 32 * 2**15 + 1])
+def test_size_rules_on_a_closed_mesh(snch, n):
+    s = scene(snch, 5)
+    p, f = points(n, seed=7)
+    same(*both_forms(snch, s, lambda: s.query_nearest(p) + s.query_silhouette(p, f)))
+
+
+def test_seeded_small_batches(snch):
+    import torch
+    s = scene(snch, 4)
+    p, f = points(5000, seed=3)
+    i, d = s.query_nearest(p)
+    sd, e = s.query_silhouette(p, f)
+    for scale in (0.5, 1.0, 2.0):  # below, at and above the answers
+        rn = torch.nextafter(d * scale, torch.full_like(d, float("inf")))
+        rs = torch.nextafter(sd * scale, torch.full_like(sd, float("inf")))
+        a, b = both_forms(snch, s, lambda: s.query_nearest_seeded(p, rn) + s.query_silhouette_seeded(p, rs, f))
+        same(a, b)
+        same(b, (i, d, sd, e))
+
+
+@pytest.mark.parametrize("n", [777, 200_000])
+def test_batched_scene(snch, n):
+    import torch
+    meshes = [mesh(k) for k in (-1, 3, 5, -2)] + [(np.zeros((0, 3), np.float32), np.zeros((0, 3), np.int32))]
+    s = snch.BatchedScene(meshes)
+    s.compute_silhouettes()
+    s.build_bvh()
+    p, f = points(n, seed=5)
+    m = torch.randint(0, len(meshes), (n,), generator=torch.Generator().manual_seed(1), dtype=torch.int32).cuda()
+    same(*both_forms(snch, s, lambda: s.query_nearest_batch(m, p) + s.query_silhouette_batch(m, p, f)))
