@@ -652,7 +652,7 @@ cudaError_t batch_view(const snch_scene_s *s, const float *keys_from, int64_t n,
     if (e != cudaSuccess)
         return e;
     uint32_t *order = nullptr;
-    e = launch_query_order(b.t, keys_from, n, b.scratch, &order, st, s->ray_order ? ray_len : nullptr);
+    e = launch_query_order(b.t, keys_from, n, b.scratch, &order, st, !ray_len, s->ray_order ? ray_len : nullptr);
     b.t.order = order;
     b.t.order_coherent = 1;
     return e;
