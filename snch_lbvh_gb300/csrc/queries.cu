@@ -58,13 +58,6 @@ SNCH_DEV float closest_point_triangle_sq(f3 pa, f3 pb, f3 pc, f3 x)
 
 SNCH_DEV float closest_point_triangle(f3 pa, f3 pb, f3 pc, f3 x) { return sqrtf(closest_point_triangle_sq(pa, pb, pc, x)); }
 
-// A candidate whose squared length s exceeds beyond(b) cannot pass a test
-// "sqrtf(s) <= b" (silhouette: b a distance) nor "sqrtf(s)^2 <= b" (nearest: b a
-// squared distance): b (1 + 2^-19), rounded twice, exceeds b (1 + 2^-20), and
-// both rounded forms of s then exceed b. So the IEEE square root is taken only
-// for candidates the exact test could accept; the answers do not change.
-SNCH_DEV float beyond_sq(float best_sq) { return best_sq * 1.0000019073486328125f; }
-
 SNCH_DEV Box load_root_box(const Box *p)
 {
     const float *q = reinterpret_cast<const float *>(p);
@@ -282,31 +275,6 @@ SNCH_DEV bool cone_overlap(const Cone &bc, f3 o, const Box &b, float dist_to_box
 // above 0.999, a query inside the bounding sphere, a margin below kConeTol) the
 // exact cone_overlap decides. A decided answer therefore equals the one the
 // reference's float arithmetic gives.
-constexpr float kConeTol = 4.0e-4f;
-constexpr float kIllCond = 0.999f;
-
-// Hardware approximations (MUFU) and fused multiply-adds: the filter only needs
-// its angles to within its margin kConeTol = 4e-4 rad, and these add a few 1e-7
-// relative (amplified at most 22.4x through arccos below kIllCond), against the
-// multi-instruction IEEE sqrtf / __frcp_rn sequences the exact path needs.
-SNCH_DEV float sqrt_approx(float x)
-{
-    float r;
-    asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
-    return r;
-}
-SNCH_DEV float rsqrt_approx(float x)
-{
-    float r;
-    asm("rsqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
-    return r;
-}
-SNCH_DEV float acos_as(float x)  // 0 <= x <= 1
-{
-    const float a0 = 1.5707288f, a1 = -0.2121144f, a2 = 0.0742610f, a3 = -0.0187293f;
-    return sqrt_approx(1.0f - x) * __fmaf_rn(x, __fmaf_rn(x, __fmaf_rn(x, a3, a2), a1), a0);
-}
-
 // 1: overlap, 0: no overlap, -1: undecided (take cone_overlap)
 SNCH_DEV int cone_overlap_fast(const Cone &bc, f3 o, const Box &b, float dist_to_box)
 {
@@ -316,35 +284,8 @@ SNCH_DEV int cone_overlap_fast(const Cone &bc, f3 o, const Box &b, float dist_to
     // measured 2 % slower: 34.44 against 33.70 ms per 16M silhouette queries)
     const f3 c = centroid(b);
     const f3 v = mk(c.x - o.x, c.y - o.y, c.z - o.z);
-    // approximate l: the asin branch below is taken only when radius / l <= kIllCond,
-    // i.e. l exceeds the radius by 0.1 %, so the exact l > radius holds there too.
-    // One reciprocal square root gives l, axis . v / l and radius / l (relative
-    // error a few 1e-7, like the square root and two divisions it replaces, which
-    // measured 1.4 % slower on the silhouette packets: 34.22 against 33.75 ms per
-    // 16M queries).
-    const float l2 = __fmaf_rn(v.x, v.x, __fmaf_rn(v.y, v.y, v.z * v.z));
-    const float rl = rsqrt_approx(l2);
-    const float l = l2 * rl;  // l2 = 0: 0 * inf = NaN, which fails the next test
-    if (!(l > 0.0f))
-        return -1;
-    const float ax = fabsf(__fmaf_rn(bc.axis.x, v.x, __fmaf_rn(bc.axis.y, v.y, bc.axis.z * v.z))) * rl;
-    if (!(ax <= kIllCond))
-        return -1;
-    const float dev = kPi2 - acos_as(ax);
-    const float ha = bc.half_angle;
-    if (dev <= ha - kConeTol)
-        return 1;
-    if (!(l > bc.radius))
-        return -1;
-    const float y = bc.radius * rl;
-    if (!(y <= kIllCond))
-        return -1;
-    const float hs = ha + (kPi2 - acos_as(fmaxf(y, 0.0f)));
-    if (hs >= kPi2 + kConeTol || dev <= hs - kConeTol)
-        return 1;
-    if (hs <= kPi2 - kConeTol && dev >= hs + kConeTol)
-        return 0;
-    return -1;
+    return cone_filter(bc.half_angle, bc.radius, __fmaf_rn(v.x, v.x, __fmaf_rn(v.y, v.y, v.z * v.z)),
+                       __fmaf_rn(bc.axis.x, v.x, __fmaf_rn(bc.axis.y, v.y, bc.axis.z * v.z)));
 }
 
 SNCH_DEV bool cone_test(const Cone &bc, f3 o, const Box &b, float dist_to_box)

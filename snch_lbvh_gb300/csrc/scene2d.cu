@@ -6,9 +6,9 @@
 //
 // Compiled with -fmad=false: every + - * / is one binary32 operation in the
 // reference's expression order, so topology, Morton codes, tree and boxes are
-// bit-identical to the reference's and the queries replay its traversal order
-// (its stack discipline and tie rules); acosf / asinf / atan2f / logf / sinf /
-// cosf are CUDA's.
+// bit-identical to the reference's; acosf / asinf / atan2f / logf / sinf / cosf
+// are CUDA's. Rays and circle samples replay the reference's traversal order; the
+// nearest and silhouette searches go near-first and give its answers (see there).
 #include <algorithm>
 #include <string>
 
@@ -150,6 +150,26 @@ SNCH_DEV float2 sv_normal(const float *verts, const int4 &sv)
     return norm2(nn);
 }
 
+// Traversal records of the nearest and silhouette searches, written by the refit and
+// the rank pass: expanding a node reads 48 consecutive bytes (80 with the cones)
+// instead of its node, two boxes and, per child, a node again (144 bytes in six
+// places); a leaf's segment and silhouette vertices are gathered in sorted order.
+struct alignas(16) Inner2
+{
+    float4 lb, rb;  // child boxes
+    uint4 ch;       // L, R, leaf info of L, of R: DFS rank | owned vertices << 30
+};
+struct Cones2
+{
+    float4 l, r;
+};
+// silhouette vertex of a leaf's segment: a = (position, unit normal of face 0),
+// b = (unit normal of face 1, bits has_face(0) | has_face(1) << 1, vertex id)
+struct Vert2
+{
+    float4 a, b;
+};
+
 // ------------------------------------------------------------------ build
 struct Build2
 {
@@ -163,7 +183,11 @@ struct Build2
     uint32_t *keys, *vals;
     NodeRec *nodes;
     float4 *aabbs, *cones;  // 2N-1 each
-    uint32_t *flags;
+    uint32_t *flags, *sizes;
+    Inner2 *inner;          // N-1
+    Cones2 *inner_cones;    // N-1
+    float4 *leaf_seg;       // N, sorted: both endpoints
+    Vert2 *leaf_verts;      // 2N: slot 2 x position + k
 };
 
 // aabb_getter scene.cuh:420-432
@@ -350,6 +374,24 @@ __global__ void __launch_bounds__(128) refit2_kernel(Build2 a)
     const uint32_t leaf = ni + j;
     a.aabbs[leaf] = a.leaf_box[orig];
     a.cones[leaf] = a.leaf_cone[orig];
+    const float2 p0 = vload2(a.verts, a.segs[2 * orig]), p1 = vload2(a.verts, a.segs[2 * orig + 1]);
+    a.leaf_seg[j] = make_float4(p0.x, p0.y, p1.x, p1.y);
+    const int2 own = a.seg_owned[orig];
+    for (int k = 0; k < 2; ++k)
+    {
+        const int32_t v = k ? own.y : own.x;
+        if (v == -1)
+            continue;
+        const int4 sv = a.sv[v];
+        const bool h0 = sv_has_face(sv, 0), h1 = sv_has_face(sv, 1);
+        const float2 pv = vload2(a.verts, sv.y);
+        const float2 n0 = h0 ? sv_face_normal(a.verts, sv, 0, true) : f2(0.0f, 0.0f);
+        const float2 n1 = h1 ? sv_face_normal(a.verts, sv, 1, true) : f2(0.0f, 0.0f);
+        Vert2 r;
+        r.a = make_float4(pv.x, pv.y, n0.x, n0.y);
+        r.b = make_float4(n1.x, n1.y, __uint_as_float((h0 ? 1u : 0u) | (h1 ? 2u : 0u)), __int_as_float(v));
+        a.leaf_verts[2 * (uint64_t)j + k] = r;
+    }
     if (n == 1)
         return;
     uint32_t cur = leaf;
@@ -370,8 +412,46 @@ __global__ void __launch_bounds__(128) refit2_kernel(Build2 a)
         m.lower = f2(fminf(lb.lower.x, rb.lower.x), fminf(lb.lower.y, rb.lower.y));
         a.aabbs[p] = pack_b2(m);
         a.cones[p] = pack_c2(cone_merge2(lc, rc, centroid2(lb), centroid2(rb), centroid2(m)));
+        a.inner[p].lb = pack_b2(lb);
+        a.inner[p].rb = pack_b2(rb);
+        a.inner_cones[p] = Cones2{pack_c2(lc), pack_c2(rc)};
         cur = p;
     }
+}
+
+// Each leaf's position in the reference's full depth-first order (leaf children of an
+// expanded node left then right, then the right subtree, then the left one), into its
+// parent's record; the near-first searches resolve exact ties with it.
+__global__ void __launch_bounds__(256) rank2_kernel(Build2 a)
+{
+    const uint32_t n = a.n, ni = n - 1;
+    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j >= n)
+        return;
+    if (j < ni)  // the child ids of internal node j
+        *reinterpret_cast<uint2 *>(&a.inner[j].ch) = make_uint2(a.nodes[j].left, a.nodes[j].right);
+    uint32_t node = ni + j, r = 0, parent = kInvalid;
+    for (int level = 0; level < 96; ++level)
+    {
+        const uint32_t p = a.nodes[node].parent;
+        if (p >= ni)
+            break;
+        if (level == 0)
+            parent = p;
+        const uint32_t L = a.nodes[p].left, R = a.nodes[p].right;
+        const uint32_t lleaf = L >= ni ? 1u : 0u, rleaf = R >= ni ? 1u : 0u;
+        if (node == L)
+            r += lleaf ? 0u : rleaf + (rleaf ? 0u : a.sizes[R]);
+        else
+            r += lleaf;
+        node = p;
+    }
+    if (parent == kInvalid)
+        return;
+    const uint32_t orig = a.vals[j];
+    const int2 own = orig < n ? a.seg_owned[orig] : make_int2(-1, -1);
+    const uint32_t info = (r & kLeafRankMask) | (uint32_t)((own.x != -1) + (own.y != -1)) << 30;
+    reinterpret_cast<uint32_t *>(&a.inner[parent].ch)[a.nodes[parent].left == ni + j ? 2 : 3] = info;
 }
 
 // ------------------------------------------------------------------ queries
@@ -384,8 +464,28 @@ struct Tree2
     const int2 *seg_owned;
     const NodeRec *nodes;
     const float4 *aabbs, *cones;
+    const Inner2 *inner;
+    const Cones2 *inner_cones;
+    const float4 *leaf_seg;
+    const Vert2 *leaf_verts;
+    const uint32_t *order;  // original segment of each sorted position
     uint32_t *status;
 };
+SNCH_DEV B2 unpack_b2(float4 v)
+{
+    B2 b;
+    b.upper = f2(v.x, v.y);
+    b.lower = f2(v.z, v.w);
+    return b;
+}
+SNCH_DEV C2 unpack_c2(float4 v)
+{
+    C2 c;
+    c.axis = f2(v.x, v.y);
+    c.half_angle = v.z;
+    c.radius = v.w;
+    return c;
+}
 SNCH_DEV B2 node_box2(const Tree2 &t, uint32_t i)
 {
     const float4 v = __ldg(t.aabbs + i);
@@ -393,15 +493,6 @@ SNCH_DEV B2 node_box2(const Tree2 &t, uint32_t i)
     b.upper = f2(v.x, v.y);
     b.lower = f2(v.z, v.w);
     return b;
-}
-SNCH_DEV C2 node_cone2(const Tree2 &t, uint32_t i)
-{
-    const float4 v = __ldg(t.cones + i);
-    C2 c;
-    c.axis = f2(v.x, v.y);
-    c.half_angle = v.z;
-    c.radius = v.w;
-    return c;
 }
 // mindist / minmaxdist aabb.cuh:130-135, 161-180
 SNCH_DEV float mindist2(const B2 &b, float2 p)
@@ -429,28 +520,52 @@ SNCH_DEV float minmaxdist2(const B2 &b, float2 p)
     }
     return fminf(rmx + rMy, rMx + rmy);
 }
-// find_closest_point_line_segment(float2) scene.cuh:176-199
-SNCH_DEV float closest_point_segment2(float2 pa, float2 pb, float2 x)
+// find_closest_point_line_segment(float2) scene.cuh:176-199: the squared length whose
+// square root is the distance
+SNCH_DEV float closest_point_segment2_sq(float2 pa, float2 pb, float2 x)
 {
     const float2 u = sub2(pb, pa), v = sub2(x, pa);
     const float c1 = dot2(u, v);
     if (c1 <= 0.0f)
-        return len2(sub2(x, pa));
+        return dot2(v, v);
     const float c2 = dot2(u, u);
     if (c2 <= c1)
-        return len2(sub2(x, pb));
+    {
+        const float2 w = sub2(x, pb);
+        return dot2(w, w);
+    }
     const float t = c1 / c2;
     const float2 pt = f2(pa.x + u.x * t, pa.y + u.y * t);
-    return len2(f2(x.x - pt.x, x.y - pt.y));
-}
-SNCH_DEV float seg_distance(const Tree2 &t, uint32_t obj, float2 p)
-{
-    return closest_point_segment2(vload2(t.verts, t.segs[2 * obj]), vload2(t.verts, t.segs[2 * obj + 1]), p);
+    const float2 w = f2(x.x - pt.x, x.y - pt.y);
+    return dot2(w, w);
 }
 SNCH_DEV float2 load_pt2(const float *p, int64_t q) { return f2(__ldg(p + 2 * q), __ldg(p + 2 * q + 1)); }
 
-// query_device(nearest) query.cuh:239-318 over segments, the reference's order;
-// a one-segment tree (where the reference reads past its node array) evaluates its leaf
+// query_device(nearest) query.cuh:239-318 over segments, near-first. The reference
+// visits its stack in a fixed order; its answer is the minimum over the leaves its
+// child tests (mindist against the sibling's minmaxdist) let it reach, the last one
+// visited among equals. Those tests depend on the node and the query alone and are
+// kept (a 2D box is inflated by 1e-3, so that the sibling test can cut off a nearer
+// segment: dropping it would change answers); pruning by the best so far never
+// removes a leaf at the minimum, so any order reaches the same minimum, and equals
+// are resolved by leaf rank. Bound by dependent reads, one record a step:
+// 180,000 segments, 200k queries 2.26 -> 0.18 ms.
+SNCH_DEV void leaf_nearest2(const Tree2 &t, uint32_t pos, uint32_t rank, float2 p, float &best, uint32_t &best_rank,
+                            uint32_t &best_pos)
+{
+    const float4 g = __ldg(t.leaf_seg + pos);
+    const float sq = closest_point_segment2_sq(f2(g.x, g.y), f2(g.z, g.w), p);
+    if (sq > beyond_sq(best))
+        return;  // d > best
+    float d = sqrtf(sq);
+    d *= d;
+    if (d < best || (d == best && (best_pos == kInvalid || rank > best_rank)))
+    {
+        best = d;
+        best_rank = rank;
+        best_pos = pos;
+    }
+}
 __global__ void __launch_bounds__(128) nearest2_kernel(Tree2 t, const float *__restrict__ pts, int64_t n,
                                                        uint32_t *__restrict__ out_idx, float *__restrict__ out_dist)
 {
@@ -458,62 +573,66 @@ __global__ void __launch_bounds__(128) nearest2_kernel(Tree2 t, const float *__r
     if (q >= n)
         return;
     const float2 p = load_pt2(pts, q);
-    uint32_t nearest = kInvalid;
+    uint32_t best_pos = kInvalid, best_rank = 0;
     float best = INFINITY;
+    const uint32_t ni = t.n - 1;
     if (t.n == 1)
-    {
-        const float d = seg_distance(t, t.nodes[0].object, p);
-        best = d * d;
-        nearest = t.nodes[0].object;
-    }
+        leaf_nearest2(t, 0u, 0u, p, best, best_rank, best_pos);
     else if (t.n > 1)
     {
         uint32_t sn[kStackDepth];
         float sd[kStackDepth];
         int sp = 0;
-        sn[sp] = 0;
-        sd[sp++] = mindist2(node_box2(t, 0), p);
-        do
+        uint32_t node = 0;
+        bool live = true;
+        while (live)
         {
-            --sp;
-            const uint32_t node = sn[sp];
-            if (sd[sp] > best)
-                continue;
-            const uint32_t ch[2] = {t.nodes[node].left, t.nodes[node].right};
-            const B2 lb = node_box2(t, ch[0]), rb = node_box2(t, ch[1]);
-            const float md[2] = {mindist2(lb, p), mindist2(rb, p)};
-            const bool ok[2] = {md[0] <= minmaxdist2(rb, p), md[1] <= minmaxdist2(lb, p)};
-            for (int k = 0; k < 2; ++k)
+            const Inner2 *rec = t.inner + node;
+            const B2 lb = unpack_b2(__ldg(&rec->lb)), rb = unpack_b2(__ldg(&rec->rb));
+            const uint4 ch = __ldg(&rec->ch);
+            const uint32_t L = ch.x, R = ch.y;
+            const float Lmd = mindist2(lb, p), Rmd = mindist2(rb, p);
+            const bool aL = Lmd <= minmaxdist2(rb, p), aR = Rmd <= minmaxdist2(lb, p);
+            if (aL && L >= ni && Lmd <= best)
+                leaf_nearest2(t, L - ni, ch.z & kLeafRankMask, p, best, best_rank, best_pos);
+            if (aR && R >= ni && Rmd <= best)
+                leaf_nearest2(t, R - ni, ch.w & kLeafRankMask, p, best, best_rank, best_pos);
+            const bool pL = aL && L < ni && Lmd <= best, pR = aR && R < ni && Rmd <= best;
+            if (pL && pR)
             {
-                if (!ok[k])
-                    continue;
-                const uint32_t obj = t.nodes[ch[k]].object;
-                if (obj != kInvalid)
+                if (sp > kStackDepth - 2)
                 {
-                    float d = seg_distance(t, obj, p);
-                    d *= d;
-                    if (d <= best)
-                    {
-                        best = d;
-                        nearest = obj;
-                    }
+                    atomicOr(t.status, kStatusStackOverflow);
+                    best_pos = kInvalid;
+                    best = NAN;
+                    break;
                 }
-                else
+                const bool l_first = Lmd <= Rmd;
+                sn[sp] = l_first ? R : L;
+                sd[sp] = l_first ? Rmd : Lmd;
+                ++sp;
+                node = l_first ? L : R;
+                continue;
+            }
+            if (pL || pR)
+            {
+                node = pL ? L : R;
+                continue;
+            }
+            live = false;
+            while (sp > 0)
+            {
+                --sp;
+                if (!(sd[sp] > best))
                 {
-                    if (sp >= kStackDepth)
-                    {
-                        atomicOr(t.status, kStatusStackOverflow);
-                        out_idx[q] = kInvalid;
-                        out_dist[q] = NAN;
-                        return;
-                    }
-                    sn[sp] = ch[k];
-                    sd[sp++] = md[k];
+                    node = sn[sp];
+                    live = true;
+                    break;
                 }
             }
-        } while (sp > 0);
+        }
     }
-    out_idx[q] = nearest;
+    out_idx[q] = best_pos == kInvalid ? kInvalid : __ldg(t.order + best_pos);
     out_dist[q] = sqrtf(best);
 }
 
@@ -533,37 +652,31 @@ SNCH_DEV bool is_silhouette_vertex(float2 n0, float2 n1, float2 view_dir, float 
     return dot0 * dot1 < 0.0f;
 }
 // silhouette_distance_calculator scene.cuh:512-532 with
-// find_closest_silhouette_point scene.cuh:354-381 per owned vertex
-SNCH_DEV bool leaf_silhouette2(const Tree2 &t, uint32_t obj, float2 o, float max_r2, float &dist, bool flip,
-                               int32_t &vid)
+// find_closest_silhouette_point scene.cuh:354-381 for one owned vertex; key = rank * 4 +
+// slot orders candidates like the reference's visits: among equal distances the last
+// one, except at distance 0, after which no vertex is accepted (the first)
+SNCH_DEV void vertex_candidate2(const Tree2 &t, uint64_t slot, uint32_t key, float2 o, bool flip, float &best,
+                                uint32_t &best_key, int32_t &best_vert)
 {
-    const int2 own = t.seg_owned[obj];
-    const int32_t ow[2] = {own.x, own.y};
-    float mr2 = max_r2;
-    bool ret = false;
-    for (int i = 0; i < 2; ++i)
+    const Vert2 *r = t.leaf_verts + slot;
+    const float4 a = __ldg(&r->a), b = __ldg(&r->b);
+    const float2 vd = f2(o.x - a.x, o.y - a.y);
+    const float sq = dot2(vd, vd);
+    if (sq > beyond_sq(best * best))
+        return;  // d > best
+    const float d = sqrtf(sq);
+    if (!(d <= best))
+        return;
+    const bool is_sil = __float_as_uint(b.z) != 3u ||
+                        is_silhouette_vertex(f2(a.z, a.w), f2(b.x, b.y), vd, d, flip);
+    if (!is_sil)
+        return;
+    if (d < best || best_vert < 0 || (d > 0.0f ? key > best_key : key < best_key))
     {
-        if (ow[i] == -1 || 0.0f >= mr2)
-            continue;
-        const int4 sv = t.sv[ow[i]];
-        const float2 pv = vload2(t.verts, sv.y);
-        const float2 vd = f2(o.x - pv.x, o.y - pv.y);
-        const float d = len2(vd);
-        if (d * d > mr2)
-            continue;
-        bool is_sil = !sv_has_face(sv, 0) || !sv_has_face(sv, 1);
-        if (!is_sil)
-            is_sil = is_silhouette_vertex(sv_face_normal(t.verts, sv, 0, true), sv_face_normal(t.verts, sv, 1, true),
-                                          vd, d, flip);
-        if (is_sil && d * d <= mr2)
-        {
-            dist = d;
-            ret = true;
-            mr2 = d * d;
-            vid = ow[i];
-        }
+        best = d;
+        best_key = key;
+        best_vert = __float_as_int(b.w);
     }
-    return ret;
 }
 // overlap(cone<float,2>) cone.cuh:78-120 with project_to_plane(float2) 44-49
 SNCH_DEV bool cone_overlap2(const C2 &bc, float2 o, const B2 &b, float dist_to_box)
@@ -592,8 +705,21 @@ SNCH_DEV bool cone_overlap2(const C2 &bc, float2 o, const B2 &b, float dist_to_b
     const float hs = bc.half_angle + atan2f(d, s);
     return hs >= kPi2 ? true : (kPi2 >= dax - hs && kPi2 <= dax + hs);
 }
-// query_device(nearest_silhouette) query.cuh:326-423 over segments, the
-// reference's order; also the silhouette vertex (mesh vertex id) of the answer
+// the same decision, mostly from the filter (cone_filter)
+SNCH_DEV bool cone_test2(const C2 &bc, float2 o, const B2 &b, float dist_to_box)
+{
+    if (bc.half_angle >= kPi2 || dist_to_box < kEps)
+        return true;
+    const float2 c = centroid2(b);
+    const float2 v = f2(c.x - o.x, c.y - o.y);
+    const int f = cone_filter(bc.half_angle, bc.radius, __fmaf_rn(v.x, v.x, v.y * v.y),
+                              __fmaf_rn(bc.axis.x, v.x, bc.axis.y * v.y));
+    return f >= 0 ? f == 1 : cone_overlap2(bc, o, b, dist_to_box);
+}
+// query_device(nearest_silhouette) query.cuh:326-423 over segments, near-first (as
+// nearest2_kernel: the cone tests alone decide which leaves can be reached); also the
+// silhouette vertex (mesh vertex id) of the answer. 180,000 segments, 200k queries
+// 46.8 -> 0.49 ms.
 __global__ void __launch_bounds__(128) silhouette2_kernel(Tree2 t, const float *__restrict__ pts,
                                                           const uint8_t *__restrict__ flips, int64_t n,
                                                           float *__restrict__ out_dist, int32_t *__restrict__ out_vid)
@@ -604,68 +730,83 @@ __global__ void __launch_bounds__(128) silhouette2_kernel(Tree2 t, const float *
     const float2 p = load_pt2(pts, q);
     const bool flip = flips ? __ldg(flips + q) != 0 : false;
     float best = INFINITY;
-    int32_t bv = -1;
+    uint32_t best_key = 0;
+    int32_t best_vert = -1;
+    const uint32_t ni = t.n - 1;
     if (t.n == 1)
     {
-        float d = INFINITY;
-        int32_t v = -1;
-        if (leaf_silhouette2(t, t.nodes[0].object, p, best * best, d, flip, v) && d <= best)
-        {
-            best = d;
-            bv = v;
-        }
+        const int2 own = t.seg_owned[t.nodes[0].object];
+        for (uint32_t k = 0; k < 2; ++k)
+            if ((k ? own.y : own.x) != -1)
+                vertex_candidate2(t, k, k, p, flip, best, best_key, best_vert);
     }
     else if (t.n > 1)
     {
         uint32_t sn[kStackDepth];
         float sd[kStackDepth];
         int sp = 0;
-        sn[sp] = 0;
-        sd[sp++] = mindist2(node_box2(t, 0), p);
-        do
+        uint32_t node = 0;
+        bool live = true;
+        while (live)
         {
-            --sp;
-            const uint32_t node = sn[sp];
-            if (sd[sp] > best * best)
-                continue;
-            const uint32_t ch[2] = {t.nodes[node].left, t.nodes[node].right};
-            for (int k = 0; k < 2; ++k)
+            const Inner2 *rec = t.inner + node;
+            const Cones2 *cr = t.inner_cones + node;
+            const B2 lb = unpack_b2(__ldg(&rec->lb)), rb = unpack_b2(__ldg(&rec->rb));
+            const uint4 ch = __ldg(&rec->ch);
+            const C2 lc = unpack_c2(__ldg(&cr->l)), rc = unpack_c2(__ldg(&cr->r));
+            const uint32_t L = ch.x, R = ch.y;
+            const float Lmd = mindist2(lb, p), Rmd = mindist2(rb, p);
+            const float b2 = best * best;
+            const bool hitL = Lmd <= b2 && lc.half_angle >= 0.0f && cone_test2(lc, p, lb, Lmd);
+            const bool hitR = Rmd <= b2 && rc.half_angle >= 0.0f && cone_test2(rc, p, rb, Rmd);
+            const uint32_t nL = hitL && L >= ni ? ch.z >> 30 : 0u, nR = hitR && R >= ni ? ch.w >> 30 : 0u;
+            for (uint32_t k = 0; k < nL + nR; ++k)
             {
-                const B2 b = node_box2(t, ch[k]);
-                const C2 c = node_cone2(t, ch[k]);
-                const float md = mindist2(b, p);
-                if (!(c.half_angle >= 0.0f && cone_overlap2(c, p, b, md)))
-                    continue;
-                const uint32_t obj = t.nodes[ch[k]].object;
-                if (obj != kInvalid)
+                const bool right = k >= nL;
+                const uint32_t slot = right ? k - nL : k;
+                vertex_candidate2(t, 2 * (uint64_t)(right ? R - ni : L - ni) + slot,
+                                  ((right ? ch.w : ch.z) & kLeafRankMask) * 4u + slot, p, flip, best, best_key,
+                                  best_vert);
+            }
+            const float b2n = best * best;
+            const bool pL = hitL && L < ni && Lmd <= b2n, pR = hitR && R < ni && Rmd <= b2n;
+            if (pL && pR)
+            {
+                if (sp > kStackDepth - 2)
                 {
-                    float d = INFINITY;
-                    int32_t v = -1;
-                    if (leaf_silhouette2(t, obj, p, best * best, d, flip, v) && d <= best)
-                    {
-                        best = d;
-                        bv = v;
-                    }
+                    atomicOr(t.status, kStatusStackOverflow);
+                    best = NAN;
+                    best_vert = -1;
+                    break;
                 }
-                else
+                const bool l_first = Lmd <= Rmd;
+                sn[sp] = l_first ? R : L;
+                sd[sp] = l_first ? Rmd : Lmd;
+                ++sp;
+                node = l_first ? L : R;
+                continue;
+            }
+            if (pL || pR)
+            {
+                node = pL ? L : R;
+                continue;
+            }
+            live = false;
+            while (sp > 0)
+            {
+                --sp;
+                if (!(sd[sp] > best * best))
                 {
-                    if (sp >= kStackDepth)
-                    {
-                        atomicOr(t.status, kStatusStackOverflow);
-                        out_dist[q] = NAN;
-                        if (out_vid)
-                            out_vid[q] = -1;
-                        return;
-                    }
-                    sn[sp] = ch[k];
-                    sd[sp++] = md;
+                    node = sn[sp];
+                    live = true;
+                    break;
                 }
             }
-        } while (sp > 0);
+        }
     }
     out_dist[q] = best;
     if (out_vid)
-        out_vid[q] = bv;
+        out_vid[q] = best_vert;
 }
 
 // intersects_d(ray<float,2>) aabb.cuh:366-390
@@ -919,11 +1060,16 @@ struct snch_scene2_s
     uint32_t *keys = nullptr, *vals = nullptr, *keys_tmp = nullptr, *vals_tmp = nullptr, *flags = nullptr,
              *sizes = nullptr, *small = nullptr;
     NodeRec *nodes = nullptr;
+    Inner2 *inner = nullptr;
+    Cones2 *inner_cones = nullptr;
+    float4 *leaf_seg = nullptr;
+    Vert2 *leaf_verts = nullptr;
     void *scratch = nullptr;
     bool built = false;
     Tree2 tree() const
     {
-        return Tree2{n, verts, segs, sv, seg_owned, nodes, aabbs, cones, small + 8};
+        return Tree2{n, verts, segs, sv, seg_owned, nodes, aabbs, cones, inner, inner_cones, leaf_seg, leaf_verts,
+                     vals, small + 8};
     }
 };
 
@@ -944,7 +1090,7 @@ void free2(snch_scene2_s *s)
 {
     void *ptrs[] = {s->verts, s->segs, s->sv, s->seg_owned, s->topo, s->leaf_box, s->leaf_cone, s->aabbs,
                     s->cones, s->keys, s->vals, s->keys_tmp, s->vals_tmp, s->flags, s->sizes, s->small,
-                    s->nodes, s->scratch};
+                    s->nodes, s->inner, s->inner_cones, s->leaf_seg, s->leaf_verts, s->scratch};
     for (void *p : ptrs)
         if (p)
             cudaFree(p);
@@ -1012,6 +1158,10 @@ int snch_scene2_create(const float *verts_xy, int64_t nv, const int32_t *segs, i
     A(dalloc2(&s->sizes, n));
     A(dalloc2(&s->small, 1056));
     A(dalloc2(&s->nodes, nn));
+    A(dalloc2(&s->inner, n));
+    A(dalloc2(&s->inner_cones, n));
+    A(dalloc2(&s->leaf_seg, n));
+    A(dalloc2(&s->leaf_verts, 2 * n));
     if (e == cudaSuccess)
         e = cudaMalloc(&s->scratch, std::max<size_t>(sort_scratch_bytes((uint32_t)std::max<size_t>(n, 1), 30), 256));
     if (e == cudaSuccess)
@@ -1065,7 +1215,8 @@ int snch_scene2_build(snch_scene2_t s, snch_stream_t stream)
     if (n)
     {
         Build2 a{n, s->verts, s->segs, s->sv, s->seg_owned, s->small, s->leaf_box, s->leaf_cone, s->keys, s->vals,
-                 s->nodes, s->aabbs, s->cones, s->flags};
+                 s->nodes, s->aabbs, s->cones, s->flags, s->sizes, s->inner, s->inner_cones, s->leaf_seg,
+                 s->leaf_verts};
         init2_kernel<<<1, 32, 0, st>>>(s->small);
         leaf2_kernel<<<blocks(n, 256), 256, 0, st>>>(a);
         morton2_kernel<<<blocks(n, 256), 256, 0, st>>>(a);
@@ -1083,7 +1234,8 @@ int snch_scene2_build(snch_scene2_t s, snch_stream_t stream)
         if (n > 1)
             SNCH2_CUDA(cudaMemsetAsync(s->flags, 0, 4 * (size_t)(n - 1), st));
         refit2_kernel<<<blocks(n, 128), 128, 0, st>>>(a);
-        note_launch();
+        rank2_kernel<<<blocks(n, 256), 256, 0, st>>>(a);
+        note_launch(2);
         SNCH2_CUDA(cudaGetLastError());
     }
     s->built = true;
