@@ -8,9 +8,10 @@
 //   karras_kernel       internal nodes (bvh.cuh:109-229) with the reference's node
 //                       numbering; ties of equal codes broken by the sorted object
 //                       index exactly as the 64-bit (code << 32 | idx) keys do
-//   refit_kernel        one bottom-up pass per leaf with atomic arrival counters that
-//                       merges AABBs (bvh.cuh:520-554) AND normal cones (bvh.cuh:559-604,
-//                       cone.cuh:427-480) and packs the 64-B traversal records
+//   leaf_records_kernel, refit_kernel, refit_top_kernel
+//                       one bottom-up pass that merges AABBs (bvh.cuh:520-554) AND normal
+//                       cones (bvh.cuh:559-604, cone.cuh:427-480) and packs the 64-B
+//                       traversal records, with the leaves' depth-first ranks
 #include <algorithm>
 
 #include "internal.h"
@@ -350,6 +351,13 @@ __global__ void __launch_bounds__(256) karras_kernel(BuildArgs a)
     nodes[ni + idx].object = a.vals[idx];
     if (idx == 0)
         nodes[0].parent = kInvalid;
+    if (a.flags)  // the 3D build: nothing has reached a node yet (refit_top_kernel)
+    {
+        if (idx < ni)
+            a.flags[idx] = 0;
+        if (idx == 0)
+            reinterpret_cast<uint32_t *>(a.centroids)[2 * (uint64_t)n] = 0;  // RefitScratch::count
+    }
     if (a.num_meshes)
     {
         // a one-triangle mesh: its root is its leaf
@@ -384,8 +392,8 @@ __global__ void __launch_bounds__(256) karras_kernel(BuildArgs a)
     nodes[right].parent = idx;
 }
 
-// silhouette_edge::normal(f, normalize) scene.cuh:745-771
-SNCH_DEV f3 edge_face_normal(const float *verts, const int4 &se, int f, bool do_normalize)
+// silhouette_edge::normal(f, normalize) scene.cuh:745-771, not normalised
+SNCH_DEV f3 edge_face_normal(const float *verts, const int4 &se, int f)
 {
     int32_t vi, vj, vk;
     if (f == 0)
@@ -401,8 +409,7 @@ SNCH_DEV f3 edge_face_normal(const float *verts, const int4 &se, int f, bool do_
         vk = se.y;
     }
     const f3 pa = load_vert(verts, vj), pb = load_vert(verts, vk), pc = load_vert(verts, vi);
-    const f3 n = cross3(sub(pb, pa), sub(pc, pa));
-    return do_normalize ? normalize3(n) : n;
+    return cross3(sub(pb, pa), sub(pc, pa));
 }
 
 // cone_getter scene.cuh:887-961 for one triangle; also emits the traversal
@@ -415,26 +422,47 @@ SNCH_DEV Cone leaf_cone(const BuildArgs &a, uint32_t orig, const Box &b, uint32_
     r.half_angle = kPi;
     r.radius = 0.0f;
     bool any = false, all_two = true;
-    int4 se[3];
+    f3 fn[3][2];  // unit face normals of the owned edges (zero where there is no face)
     n_owned = 0;
+    int32_t own[3];
+    int4 ev[3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+        own[i] = __ldg(a.tri_owned + 3 * (uint64_t)orig + i);
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+        if ((uint32_t)own[i] < 3 * a.num_tris)
+            ev[i] = __ldg(reinterpret_cast<const int4 *>(a.edge_verts) + own[i]);
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+        if ((uint32_t)own[i] < 3 * a.num_tris)
+        {
+            if (ev[i].x != -1)
+                asm volatile("prefetch.global.L1 [%0];" ::"l"(a.verts + 3 * (int64_t)ev[i].x));
+            if (ev[i].w != -1)
+                asm volatile("prefetch.global.L1 [%0];" ::"l"(a.verts + 3 * (int64_t)ev[i].w));
+        }
+#pragma unroll
     for (int i = 0; i < 3; ++i)
     {
-        const int32_t s = __ldg(a.tri_owned + 3 * (uint64_t)orig + i);
-        if (s < 0 || (uint32_t)s >= 3 * a.num_tris)
+        const int32_t s = own[i];
+        if ((uint32_t)s >= 3 * a.num_tris)
             continue;
-        const int4 e = __ldg(reinterpret_cast<const int4 *>(a.edge_verts) + s);
+        const int4 e = ev[i];
         const bool h0 = e.w != -1, h1 = e.x != -1;  // has_face(0), has_face(1) scene.cuh:741-744
         // silhouette_edge::normal() scene.cuh:772-786
-        f3 nsum = mk(0.0f, 0.0f, 0.0f);
+        f3 nsum = mk(0.0f, 0.0f, 0.0f), fn0 = nsum, fn1 = nsum;
         if (h0)
         {
-            const f3 n0 = edge_face_normal(a.verts, e, 0, false);
+            const f3 n0 = edge_face_normal(a.verts, e, 0);
             nsum = mk(nsum.x + n0.x, nsum.y + n0.y, nsum.z + n0.z);
+            fn0 = normalize3(n0);
         }
         if (h1)
         {
-            const f3 n1 = edge_face_normal(a.verts, e, 1, false);
+            const f3 n1 = edge_face_normal(a.verts, e, 1);
             nsum = mk(nsum.x + n1.x, nsum.y + n1.y, nsum.z + n1.z);
+            fn1 = normalize3(n1);
         }
         const f3 sn = normalize3(nsum);
         r.axis.x += sn.x;
@@ -446,15 +474,19 @@ SNCH_DEV Cone leaf_cone(const BuildArgs &a, uint32_t orig, const Box &b, uint32_
         all_two = all_two && h0 && h1;
         any = true;
         // traversal record of this owned edge
-        const f3 fn0 = h0 ? edge_face_normal(a.verts, e, 0, true) : mk(0.0f, 0.0f, 0.0f);
-        const f3 fn1 = h1 ? edge_face_normal(a.verts, e, 1, true) : mk(0.0f, 0.0f, 0.0f);
         EdgeRec er;
         er.a = make_float4(pa.x, pa.y, pa.z, __uint_as_float((h0 ? 1u : 0u) | (h1 ? 2u : 0u)));
         er.b = make_float4(pb.x, pb.y, pb.z, __int_as_float(s));
         er.c = make_float4(fn0.x, fn0.y, fn0.z, 0.0f);
         er.d = make_float4(fn1.x, fn1.y, fn1.z, 0.0f);
         a.edges[3 * (uint64_t)pos + n_owned] = er;
-        se[n_owned] = e;
+#pragma unroll
+        for (int k = 0; k < 3; ++k)  // constant indices: the array stays in registers
+            if (k == (int)n_owned)
+            {
+                fn[k][0] = fn0;
+                fn[k][1] = fn1;
+            }
         ++n_owned;
     }
     if (!any)
@@ -470,17 +502,13 @@ SNCH_DEV Cone leaf_cone(const BuildArgs &a, uint32_t orig, const Box &b, uint32_
             r.axis.y /= axis_norm;
             r.axis.z /= axis_norm;
             r.half_angle = 0.0f;
-            for (uint32_t i = 0; i < n_owned; ++i)
-            {
-                const bool h0 = se[i].w != -1, h1 = se[i].x != -1;
-                const f3 fn[2] = {h0 ? edge_face_normal(a.verts, se[i], 0, true) : mk(0.0f, 0.0f, 0.0f),
-                                  h1 ? edge_face_normal(a.verts, se[i], 1, true) : mk(0.0f, 0.0f, 0.0f)};
-                for (int j = 0; j < 2; ++j)
+#pragma unroll
+            for (int i = 0; i < 3; ++i)
+                for (int j = 0; j < 2 && i < (int)n_owned; ++j)
                 {
-                    const float angle = acosf(smax(-1.0f, smin(1.0f, dot3(r.axis, fn[j]))));
+                    const float angle = acosf(smax(-1.0f, smin(1.0f, dot3(r.axis, fn[i][j]))));
                     r.half_angle = smax(r.half_angle, angle);
                 }
-            }
         }
     }
     return r;
@@ -501,7 +529,8 @@ SNCH_DEV f3 rotate3(f3 u, f3 v, float theta)
 // merge(cone, cone, origins) cone.cuh:427-480; where the reference leaves
 // half_angle unassigned (o_theta >= pi, 454-458) the conservative pi is stored,
 // and a merge of two invalid cones gets a zero axis and radius.
-SNCH_DEV Cone cone_merge(const Cone &a, const Cone &b, f3 oa, f3 ob, f3 on)
+// da2, db2: squared distances of the merged box's centroid from the children's
+SNCH_DEV Cone cone_merge(const Cone &a, const Cone &b, float da2, float db2)
 {
     Cone r;
     r.axis = mk(0.0f, 0.0f, 0.0f);
@@ -512,8 +541,7 @@ SNCH_DEV Cone cone_merge(const Cone &a, const Cone &b, f3 oa, f3 ob, f3 on)
     {
         f3 axis_a = a.axis, axis_b = b.axis;
         float ha = a.half_angle, hb = b.half_angle;
-        const f3 da = sub(on, oa), db = sub(on, ob);
-        r.radius = sqrtf(smax(a.radius * a.radius + sqlen3(da), b.radius * b.radius + sqlen3(db)));
+        r.radius = sqrtf(smax(a.radius * a.radius + da2, b.radius * b.radius + db2));
         if (hb > ha)
         {
             const f3 t = axis_a;
@@ -568,92 +596,297 @@ SNCH_DEV Cone ldcg_cone(const Cone *p)
     return c;
 }
 
-// One thread per sorted leaf: leaf box + cone + traversal records, then the
-// walk towards the root. The first thread to reach a node stops; the second
-// (whose sibling's results are published by the sibling's fence + atomic)
-// merges both children.
-__global__ void __launch_bounds__(128) refit_kernel(BuildArgs a)
+// ---- leaves to root, in three kernels
+//   leaf_records_kernel  leaf boxes, cones, traversal records and ranks
+//   refit_kernel         the nodes whose leaves all lie in one block, in shared memory
+//   refit_top_kernel     the rest, bottom-up through global memory
+// Almost every internal node covers leaves of one block of kRefitLeaves consecutive
+// ones. A Karras node's index is an end of its leaf range, so such a node has the
+// block-local slot index - first leaf.
+// One walk per leaf from its records to the root through global memory, in one kernel,
+// took 864 us for 2M triangles and the ranks 85 us in another: the walk holds its
+// block's place while one lane of it waits for fences, an atomic and three dependent
+// reads a level, and the gathers of the leaves wait for few warps. Here 250 + 204 + 74
+// us (one kernel for all three: 770 us, held up by the walks at its end).
+constexpr int kRefitLeaves = 256;
+
+// scratch in the space of the centroids, which are dead after the Morton codes
+struct RefitScratch
 {
+    uint32_t *info;   // per sorted leaf: DFS rank | owned edges << 30
+    uint32_t *exits;  // subtrees whose parent reaches into another block
+    uint32_t *count;  // of exits (cleared by karras_kernel)
+};
+SNCH_DEV RefitScratch refit_scratch(const BuildArgs &a)
+{
+    uint32_t *w = reinterpret_cast<uint32_t *>(a.centroids);
+    return RefitScratch{w, w + a.num_tris, w + 2 * (uint64_t)a.num_tris};
+}
+
+// the internal node at index j, with w = 1 if its leaves, and so the slots of its
+// children, all lie in the block of first leaf b0; size: leaves under it
+SNCH_DEV uint4 block_node(const BuildArgs &a, uint32_t j, uint32_t b0, uint32_t &size)
+{
+    constexpr uint32_t B = kRefitLeaves;
+    const uint32_t ni = a.num_tris - 1;
+    size = 0;
+    if (j >= ni)
+        return make_uint4(kInvalid, kInvalid, kInvalid, 0u);
+    uint4 node = __ldg(reinterpret_cast<const uint4 *>(a.nodes + j));  // parent, left, right, object
+    size = __ldg(a.sizes + j);
+    const uint32_t gl = node.y >= ni ? node.y - ni : node.y, gr = node.z >= ni ? node.z - ni : node.z;
+    const uint32_t lo = gl >= j ? j : j + 1u - size;  // the split lies on the range's side of its node
+    node.w = lo >= b0 && lo <= j && lo + size <= b0 + B && gl - b0 < B && gr - b0 < B ? 1u : 0u;
+    return node;
+}
+
+// Rank: a leaf's position in the reference's full depth-first visit order
+// (query.cuh:256-316): expanding node n emits its leaf children (left, then right),
+// then visits the right subtree, then the left one. It is the sum, over the path to the
+// root, of the offset of each node within its parent's emission sequence. The near-first
+// traversals resolve exact distance ties with it. Stored in LeafRec.v2.w and, with the
+// owned-edge count, in the parent's InnerRec.
+// Offset of child `node` in the emission sequence of its parent (children L, R);
+// size_r: leaves under R
+SNCH_DEV uint32_t emission_offset(uint32_t node, uint32_t L, uint32_t R, uint32_t ni, uint32_t size_r)
+{
+    const uint32_t lleaf = L >= ni ? 1u : 0u, rleaf = R >= ni ? 1u : 0u;
+    if (node == L)
+        return lleaf ? 0u : rleaf + (rleaf ? 0u : size_r);
+    return lleaf;
+}
+// the offsets of the path from a node to the root, through global memory
+SNCH_DEV uint32_t rank_base(const BuildArgs &a, uint32_t node, uint32_t parent)
+{
+    const uint32_t ni = a.num_tris - 1;
+    uint32_t r = 0, p = parent;
+    for (int level = 0; level < 96 && p < ni; ++level)
+    {
+        const uint4 rec = __ldg(reinterpret_cast<const uint4 *>(a.nodes + p));
+        r += emission_offset(node, rec.y, rec.z, ni,
+                             node == rec.y && rec.y < ni && rec.z < ni ? __ldg(a.sizes + rec.z) : 0u);
+        node = p;
+        p = rec.x;
+    }
+    return r;
+}
+
+// Bound by the latency of its gathers (triangle, its corners, its owned edges, their
+// opposite corners, in Morton order): four dependent reads, so as many warps as the
+// registers allow and the last reads requested together. 2M triangles: 250 us (3 / 5 / 6
+// blocks per SM: 288 / 261 / 273), about 1 GB of sectors.
+__global__ void __launch_bounds__(kRefitLeaves, 4) leaf_records_kernel(BuildArgs a)
+{
+    constexpr uint32_t B = kRefitLeaves;
+    __shared__ uint4 s_node[B];
+    __shared__ uint32_t s_size[B], s_base[2 * B];
     const uint32_t n = a.num_tris, ni = n - 1;
-    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n)
+    const uint32_t b0 = blockIdx.x * B, t = threadIdx.x, j = b0 + t;
+    const auto inside = [&](uint32_t p) { return p - b0 < B && s_node[p - b0].w != 0u; };  // p may be kInvalid
+    const uint32_t orig = j < n ? __ldg(a.vals + j) : kInvalid;
+    const bool leaf = orig < n;  // otherwise past the end, or after a failed sort (status bit set)
+    const uint32_t parent = leaf && n > 1 ? a.nodes[ni + j].parent : kInvalid;
+    uint32_t size;
+    const uint4 node = block_node(a, j, b0, size);
+    s_node[t] = node;
+    s_size[t] = size;
+    __syncthreads();
+    // ranks: up to the last node inside the block, then that node's own offset, which
+    // one thread takes from global memory
+    if (node.w && !inside(node.x))
+        s_base[B + t] = rank_base(a, j, node.x);
+    uint32_t r = 0, top = t;
+    if (leaf)
+    {
+        if (!inside(parent))
+            s_base[t] = rank_base(a, ni + j, parent);
+        uint32_t cur = ni + j, p = parent;
+        for (int level = 0; level < 96 && inside(p); ++level)
+        {
+            const uint4 rec = s_node[p - b0];
+            r += emission_offset(cur, rec.y, rec.z, ni, rec.z < ni ? s_size[rec.z - b0] : 0u);
+            cur = p;
+            p = rec.x;
+            top = B + cur - b0;
+        }
+    }
+    __syncthreads();
+    if (!leaf)
         return;
-    const uint32_t orig = __ldg(a.vals + j);
-    if (orig >= n)  // only after a failed sort (status bit set)
-        return;
-    const int32_t *t = a.tris + 3 * (uint64_t)orig;
-    const f3 pa = load_vert(a.verts, __ldg(t)), pb = load_vert(a.verts, __ldg(t + 1)),
-             pc = load_vert(a.verts, __ldg(t + 2));
+    r += s_base[top];
+    const int32_t *tr = a.tris + 3 * (uint64_t)orig;
+    const f3 pa = load_vert(a.verts, __ldg(tr)), pb = load_vert(a.verts, __ldg(tr + 1)),
+             pc = load_vert(a.verts, __ldg(tr + 2));
     const Box b = tri_box(pa, pb, pc);
     uint32_t n_owned;
     const Cone c = leaf_cone(a, orig, b, j, n_owned);
-    const uint32_t leaf = ni + j;
-    a.aabbs[leaf] = b;
-    a.cones[leaf] = c;
+    a.aabbs[ni + j] = b;
+    a.cones[ni + j] = c;
     LeafRec lr;
     lr.v0 = make_float4(pa.x, pa.y, pa.z, __uint_as_float(orig));
     lr.v1 = make_float4(pb.x, pb.y, pb.z, __uint_as_float(n_owned));
-    lr.v2 = make_float4(pc.x, pc.y, pc.z, 0.0f);
+    lr.v2 = make_float4(pc.x, pc.y, pc.z, __uint_as_float(r));
     a.leaves[j] = lr;
-    if (n == 1)
-        return;
-    uint32_t cur = leaf;
-    // a Karras tree over 64-bit keys is at most 65 levels deep
-    for (int level = 0; level < 96; ++level)
-    {
-        const uint32_t p = a.nodes[cur].parent;
-        if (p >= ni)
-            return;
-        __threadfence();
-        if (atomicAdd(a.flags + p, 1u) == 0u)
-            return;
-        __threadfence();
-        const uint32_t L = a.nodes[p].left, R = a.nodes[p].right;
-        const Box lb = ldcg_box(a.aabbs + L), rb = ldcg_box(a.aabbs + R);
-        const Cone lc = ldcg_cone(a.cones + L), rc = ldcg_cone(a.cones + R);
-        const Box m = merge_box(lb, rb);
-        a.aabbs[p] = m;
-        a.cones[p] = cone_merge(lc, rc, centroid(lb), centroid(rb), centroid(m));
-        a.inner[p] = pack_inner(lb, rb, L, R);
-        a.inner_cones[p] = pack_cones(lc, rc);
-        cur = p;
-    }
+    refit_scratch(a).info[j] = (r & kLeafRankMask) | (n_owned << 30);
 }
 
-// Position of every leaf in the reference's full depth-first visit order
-// (query.cuh:256-316): expanding node n emits its leaf children (left, then
-// right), then visits the right subtree, then the left one. A leaf's position
-// is the sum, over the path to the root, of the offset of each node within its
-// parent's emission sequence. The near-first traversals use it to resolve exact
-// distance ties the way the reference's visit order does. Stored in LeafRec.v2.w.
-__global__ void __launch_bounds__(256) rank_kernel(BuildArgs a)
+// Rounds: a round's list holds the nodes whose children are both done, taken by
+// consecutive threads (the merge's acosf, sinf and cosf run in full warps; a walk per
+// leaf loses half of its lanes at every level). Bound by the chain of about 15 such merges;
+// 6 blocks per SM: 204 us, 5 / 4: 212 / 224.
+__global__ void __launch_bounds__(kRefitLeaves, 6) refit_kernel(BuildArgs a)
 {
+    constexpr uint32_t B = kRefitLeaves;
+    __shared__ float s_val[11][2 * B];  // box and cone: slot t = leaf t, B + t = internal node t
+    __shared__ uint4 s_node[B];
+    __shared__ uint32_t s_info[B], s_arrived[B], s_list[2][B], s_exit[B];
+    __shared__ uint32_t s_count[2], s_exits, s_exit_base;
     const uint32_t n = a.num_tris, ni = n - 1;
-    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n)
-        return;
-    uint32_t node = ni + j, r = 0;
-    for (int level = 0; level < 96 && n > 1; ++level)
+    const uint32_t b0 = blockIdx.x * B, t = threadIdx.x, j = b0 + t;
+    const RefitScratch scratch = refit_scratch(a);
+    const auto put_box = [&](uint32_t slot, const Box &b) {
+        const float v[6] = {b.upper.x, b.upper.y, b.upper.z, b.lower.x, b.lower.y, b.lower.z};
+#pragma unroll
+        for (int k = 0; k < 6; ++k)
+            s_val[k][slot] = v[k];
+    };
+    const auto put_cone = [&](uint32_t slot, const Cone &c) {
+        const float v[5] = {c.axis.x, c.axis.y, c.axis.z, c.half_angle, c.radius};
+#pragma unroll
+        for (int k = 0; k < 5; ++k)
+            s_val[6 + k][slot] = v[k];
+    };
+    const auto get_box = [&](uint32_t slot) {
+        Box b;
+        b.upper = mk(s_val[0][slot], s_val[1][slot], s_val[2][slot]);
+        b.lower = mk(s_val[3][slot], s_val[4][slot], s_val[5][slot]);
+        return b;
+    };
+    const auto get_cone = [&](uint32_t slot) {
+        Cone c;
+        c.axis = mk(s_val[6][slot], s_val[7][slot], s_val[8][slot]);
+        c.half_angle = s_val[9][slot];
+        c.radius = s_val[10][slot];
+        return c;
+    };
+    const auto inside = [&](uint32_t p) { return p - b0 < B && s_node[p - b0].w != 0u; };  // p may be kInvalid
+    // slot of a child of a node that is inside
+    const auto slot_of = [&](uint32_t child) { return child >= ni ? child - ni - b0 : B + child - b0; };
+    // a finished node: its parent's place in the next round's list, or an exit
+    const auto arrive = [&](uint32_t done, uint32_t p, uint32_t next) {
+        if (!inside(p))
+            s_exit[atomicAdd(&s_exits, 1u)] = done;
+        else if (atomicAdd(&s_arrived[p - b0], 1u) == 1u)
+            s_list[next][atomicAdd(&s_count[next], 1u)] = p - b0;
+    };
+
+    uint32_t size;
+    s_node[t] = block_node(a, j, b0, size);
+    s_arrived[t] = 0;
+    if (t < 2)
+        s_count[t] = 0;
+    if (t == 0)
+        s_exits = 0;
+    const bool leaf = j < n && __ldg(a.vals + j) < n;
+    if (leaf)
     {
-        const uint32_t p = a.nodes[node].parent;
-        if (p >= ni)
-            break;
-        const uint32_t L = a.nodes[p].left, R = a.nodes[p].right;
-        const uint32_t lleaf = L >= ni ? 1u : 0u, rleaf = R >= ni ? 1u : 0u;
-        if (node == L)
-            r += lleaf ? 0u : lleaf + rleaf + (rleaf ? 0u : a.sizes[R]);
-        else
-            r += rleaf ? lleaf : lleaf + rleaf;
-        node = p;
+        put_box(t, ldcg_box(a.aabbs + ni + j));
+        put_cone(t, ldcg_cone(a.cones + ni + j));
+        s_info[t] = scratch.info[j];
     }
-    a.leaves[j].v2.w = __uint_as_float(r);
-    // the leaf's rank and owned-edge count in its parent's traversal record
-    const uint32_t p = n > 1 ? a.nodes[ni + j].parent : kInvalid;
-    if (p < ni)
+    __syncthreads();
+    if (leaf)
+        arrive(ni + j, a.nodes[ni + j].parent, 0u);
+    __syncthreads();
+    uint32_t cur = 0;
+    while (true)
     {
-        const uint32_t info = (r & kLeafRankMask) | (__float_as_uint(a.leaves[j].v1.w) << 30);
-        float *d = reinterpret_cast<float *>(&a.inner[p].d);
-        d[a.nodes[p].left == ni + j ? 2 : 3] = __uint_as_float(info);
+        const uint32_t count = s_count[cur];
+        if (count == 0)
+            break;
+        if (t < count)
+        {
+            const uint32_t s = s_list[cur][t], p = b0 + s;
+            const uint4 rec = s_node[s];
+            // the boxes are done with before the cones are read (fewer registers, so
+            // more blocks, which hide the merge's chain of dependent operations)
+            float da2, db2;
+            {
+                const Box lb = get_box(slot_of(rec.y)), rb = get_box(slot_of(rec.z));
+                const Box m = merge_box(lb, rb);
+                const f3 cm = centroid(m);
+                da2 = sqlen3(sub(cm, centroid(lb)));
+                db2 = sqlen3(sub(cm, centroid(rb)));
+                put_box(B + s, m);
+                a.aabbs[p] = m;
+                InnerRec ir = pack_inner(lb, rb, rec.y, rec.z);
+                if (rec.y >= ni)
+                    ir.d.z = __uint_as_float(s_info[rec.y - ni - b0]);
+                if (rec.z >= ni)
+                    ir.d.w = __uint_as_float(s_info[rec.z - ni - b0]);
+                a.inner[p] = ir;
+            }
+            const Cone lc = get_cone(slot_of(rec.y)), rc = get_cone(slot_of(rec.z));
+            a.inner_cones[p] = pack_cones(lc, rc);
+            const Cone c = cone_merge(lc, rc, da2, db2);
+            put_cone(B + s, c);
+            a.cones[p] = c;
+            arrive(p, rec.x, cur ^ 1u);
+        }
+        __syncthreads();
+        if (t == 0)
+            s_count[cur] = 0;
+        cur ^= 1u;
+        __syncthreads();
+    }
+    if (t == 0)
+        s_exit_base = atomicAdd(scratch.count, s_exits);
+    __syncthreads();
+    if (t < s_exits)
+        scratch.exits[s_exit_base + t] = s_exit[t];
+}
+
+// counts an arrival; releases this thread's writes and acquires those of the arrivals before
+SNCH_DEV uint32_t arrive_acq_rel(uint32_t *p)
+{
+    uint32_t old;
+    asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(old) : "l"(p) : "memory");
+    return old;
+}
+// The first thread to reach a node stops; the second (whose sibling's results are
+// published by the sibling's arrival, or by the end of refit_kernel) merges.
+__global__ void __launch_bounds__(128) refit_top_kernel(BuildArgs a)
+{
+    const uint32_t ni = a.num_tris - 1;
+    const RefitScratch scratch = refit_scratch(a);
+    const uint32_t count = *scratch.count;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x)
+    {
+        uint32_t up = scratch.exits[i];
+        // a Karras tree over 64-bit keys is at most 65 levels deep
+        for (int level = 0; level < 96; ++level)
+        {
+            const uint32_t p = a.nodes[up].parent;
+            if (p >= ni)
+                break;
+            if (arrive_acq_rel(a.flags + p) == 0u)
+                break;
+            const uint32_t L = a.nodes[p].left, R = a.nodes[p].right;
+            const Box lb = ldcg_box(a.aabbs + L), rb = ldcg_box(a.aabbs + R);
+            const Cone lc = ldcg_cone(a.cones + L), rc = ldcg_cone(a.cones + R);
+            const Box m = merge_box(lb, rb);
+            a.aabbs[p] = m;
+            const f3 cm = centroid(m);
+            a.cones[p] = cone_merge(lc, rc, sqlen3(sub(cm, centroid(lb))), sqlen3(sub(cm, centroid(rb))));
+            InnerRec ir = pack_inner(lb, rb, L, R);
+            if (L >= ni)
+                ir.d.z = __uint_as_float(scratch.info[L - ni]);
+            if (R >= ni)
+                ir.d.w = __uint_as_float(scratch.info[R - ni]);
+            a.inner[p] = ir;
+            a.inner_cones[p] = pack_cones(lc, rc);
+            up = p;
+        }
     }
 }
 
@@ -947,16 +1180,15 @@ cudaError_t launch_build_back(const BuildArgs &a, cudaStream_t st)
     const uint32_t n = a.num_tris;
     karras_kernel<<<(n + 255) / 256, 256, 0, st>>>(a);
     note_launch();
+    const uint32_t blocks = (n + kRefitLeaves - 1) / kRefitLeaves;
+    leaf_records_kernel<<<blocks, kRefitLeaves, 0, st>>>(a);
+    note_launch();
     if (n > 1)
     {
-        cudaError_t e = cudaMemsetAsync(a.flags, 0, 4 * (size_t)(n - 1), st);
-        if (e != cudaSuccess)
-            return e;
+        refit_kernel<<<blocks, kRefitLeaves, 0, st>>>(a);
+        refit_top_kernel<<<(16 * blocks + 127) / 128, 128, 0, st>>>(a);  // about 16 exits a block
+        note_launch(2);
     }
-    refit_kernel<<<(n + 127) / 128, 128, 0, st>>>(a);
-    note_launch();
-    rank_kernel<<<(n + 255) / 256, 256, 0, st>>>(a);
-    note_launch();
     return cudaGetLastError();
 }
 
