@@ -482,8 +482,9 @@ int create_common(const float *v, int64_t nv, const int32_t *t, int64_t nt, snch
 
 int topology(snch_scene_s *s, cudaStream_t st)
 {
-    SNCH_CUDA(compute_topology(s->tris, s->num_tris, s->tri_edges, s->tri_owned, s->edge_verts,
-                               s->small + kWNumEdges, s->scratch, s->small + kWStatus, st));
+    SNCH_CUDA(compute_topology(s->tris, s->num_tris, s->num_verts, s->tri_edges, s->tri_owned, s->edge_verts,
+                               s->small + kWNumEdges, s->verts, s->ref_objects, s->ref_edges, s->scratch,
+                               s->small + kWStatus, st));
     s->topology_ready = true;
     s->num_edges_host = -1;
     return SNCH_OK;
@@ -1055,8 +1056,6 @@ int snch_build_bvh(snch_scene_t s, snch_stream_t stream)
                                    s->scratch, s->small + kWStatus, st));
         SNCH_CUDA(launch_mesh_pass(a, s->scratch, st));  // batched scenes only
         SNCH_CUDA(launch_build_back(a, st));
-        SNCH_CUDA(launch_ref_objects(s->verts, s->tris, s->tri_owned, s->edge_verts, s->num_tris, s->ref_objects,
-                                     s->ref_edges, st));
         if (s->num_meshes == 0)
             SNCH_CUDA(launch_top_levels(s->inner, s->inner_cones, s->num_tris, kTopSlots, s->top_inner,
                                         s->top_cones, st));

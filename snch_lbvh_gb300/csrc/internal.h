@@ -216,9 +216,11 @@ inline int sort_passes(int key_bits) { return (key_bits + 7) / 8; }
 
 // ---- topology.cu (scene.cuh:1135-1225 on the device)
 size_t topology_scratch_bytes(uint32_t num_tris);
-// Outputs: tri_edges, tri_owned (int32 x 3N), edge_verts (int32 x 4 x capacity 3N), *num_edges (device).
-cudaError_t compute_topology(const int32_t *tris, uint32_t num_tris, int32_t *tri_edges, int32_t *tri_owned,
-                             int32_t *edge_verts, uint32_t *num_edges, void *scratch, uint32_t *status,
+// Outputs: tri_edges, tri_owned (int32 x 3N), edge_verts (int32 x 4 x capacity 3N), *num_edges
+// (device), and the objects of the byte-compatible view, which point at verts and ref_edges.
+cudaError_t compute_topology(const int32_t *tris, uint32_t num_tris, uint32_t num_verts, int32_t *tri_edges,
+                             int32_t *tri_owned, int32_t *edge_verts, uint32_t *num_edges, const float *verts,
+                             snch_triangle *objs, snch_silhouette_edge *ref_edges, void *scratch, uint32_t *status,
                              cudaStream_t st);
 
 }  // namespace snch
