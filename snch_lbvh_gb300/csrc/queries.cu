@@ -596,6 +596,30 @@ SNCH_DEV void prefetch_l1(const void *p) { asm volatile("prefetch.global.L1 [%0]
 // for silhouettes (40.9 vs 35.6 ms per 16M queries) and 11 % for nearest, so
 // they do not prefetch either.
 
+// Queries that a launch leaves to the next one, which finishes them one per warp
+// (coop.cuh) from the candidate each has: the long packets at the end of a batch
+// (leave_packet) and the long searches of a mid-sized batch (kDefer below).
+struct DeferArgs
+{
+    uint4 *list = nullptr;      // (query, candidate's distance bits, rank or key, triangle or edge); nullptr: off
+    uint32_t *count = nullptr;  // entries reserved; may pass capacity, by entries that are not in the list
+    uint32_t capacity = 0;
+};
+// lists the entry of every lane with `add` set; called by any subset of a warp
+SNCH_DEV void defer_query(const DeferArgs &d, bool add, uint4 entry)
+{
+    const uint32_t active = __activemask(), mask = __ballot_sync(active, add);
+    if (!add)
+        return;
+    const int lane = threadIdx.x & 31, leader = __ffs(mask) - 1;
+    uint32_t base = 0;
+    if (lane == leader)
+        base = atomicAdd(d.count, (uint32_t)__popc(mask));
+    base = __shfl_sync(mask, base, leader);
+    d.list[base + __popc(mask & ((1u << lane) - 1u))] = entry;
+}
+constexpr uint32_t kLaneTurns = 32;  // expansions before a query is left to the next launch
+
 // (128, 10): at most 48 registers, ten blocks per SM (silhouette: (128, 9), 56
 // registers, nine blocks). The traversals wait on dependent L2 loads; the extra
 // resident warps hide more of that latency (measured on the 2M-triangle scene:
@@ -604,10 +628,11 @@ SNCH_DEV void prefetch_l1(const void *p) { asm volatile("prefetch.global.L1 [%0]
 // (1280 nearest, 1152 silhouette) in smaller or larger blocks. A block's slot
 // on the SM is freed only when its slowest query is done, so smaller blocks
 // lose less to the long tail of per-query work.
-template <bool kStats, int kBlock = 128>
+template <bool kStats, int kBlock = 128, bool kDefer = false>
 __global__ void __launch_bounds__(kBlock, 1280 / kBlock) nearest_fast_kernel(TreeView t, const float *__restrict__ pts, int64_t n,
                                                            uint32_t *__restrict__ out_idx, float *__restrict__ out_dist,
-                                                           uint32_t *__restrict__ stats, SeedArgs seed)
+                                                           uint32_t *__restrict__ stats, SeedArgs seed,
+                                                           DeferArgs defer = DeferArgs())
 {
     uint32_t n_int = 0, n_leaf = 0;
     const int64_t qi = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -623,7 +648,7 @@ __global__ void __launch_bounds__(kBlock, 1280 / kBlock) nearest_fast_kernel(Tre
         best = r0 * r0;
     }
     bool deferred = false;
-    uint32_t budget = seed.cap ? seed.cap : 0xFFFFFFFFu;
+    uint32_t budget = kDefer ? kLaneTurns : seed.cap ? seed.cap : 0xFFFFFFFFu;
     const uint32_t ni = t.num_tris - 1;
     const QueryRoot qr = query_root(t, q);
     if (qr.node == kInvalid)
@@ -719,7 +744,13 @@ __global__ void __launch_bounds__(kBlock, 1280 / kBlock) nearest_fast_kernel(Tre
         stats[3 * q + 1] = n_leaf;
         stats[3 * q + 2] = 0;
     }
-    if (deferred)
+    if (kDefer)
+    {
+        defer_query(defer, deferred, make_uint4((uint32_t)q, __float_as_uint(best), best_rank, nearest));
+        if (deferred)
+            return;
+    }
+    else if (deferred)
     {
         // the bound handed to the second pass: a float whose square is >= best
         seed.defer_radius[q] = best < INFINITY ? nextafterf(sqrtf(best), INFINITY) : INFINITY;
@@ -828,12 +859,13 @@ SNCH_DEV void leaf_silhouette_info(const TreeView &t, uint32_t pos, uint32_t inf
         edge_candidate(t, pos, k, rank, o, flip, best, best_key, best_edge);
 }
 
-template <bool kStats, int kBlock = 128>
+template <bool kStats, int kBlock = 128, bool kDefer = false>
 __global__ void __launch_bounds__(kBlock, 1152 / kBlock) silhouette_fast_kernel(TreeView t, const float *__restrict__ pts,
                                                               const uint8_t *__restrict__ flips, int64_t n,
                                                               float *__restrict__ out_dist,
                                                               int32_t *__restrict__ out_edge,
-                                                              uint32_t *__restrict__ stats, SeedArgs seed)
+                                                              uint32_t *__restrict__ stats, SeedArgs seed,
+                                                              DeferArgs defer = DeferArgs())
 {
     uint32_t n_int = 0, n_leaf = 0, n_edge = 0;
     const int64_t qi = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -847,7 +879,7 @@ __global__ void __launch_bounds__(kBlock, 1152 / kBlock) silhouette_fast_kernel(
     uint32_t best_key = 0;
     int32_t best_edge = -1;
     bool deferred = false;
-    uint32_t budget = seed.cap ? seed.cap : 0xFFFFFFFFu;
+    uint32_t budget = kDefer ? kLaneTurns : seed.cap ? seed.cap : 0xFFFFFFFFu;
     const uint32_t ni = t.num_tris - 1;
     const QueryRoot qr = query_root(t, q);
     if (qr.node == kInvalid)
@@ -949,7 +981,13 @@ __global__ void __launch_bounds__(kBlock, 1152 / kBlock) silhouette_fast_kernel(
             }
         }
     }
-    if (deferred)
+    if (kDefer)
+    {
+        defer_query(defer, deferred, make_uint4((uint32_t)q, __float_as_uint(best), best_key, (uint32_t)best_edge));
+        if (deferred)
+            return;
+    }
+    else if (deferred)
     {
         seed.defer_radius[q] = best;  // best candidate so far, or the seed radius
         append_failed(seed.defer_list, seed.defer_count, (uint32_t)q, true);
@@ -1481,12 +1519,6 @@ __device__ __noinline__ unsigned long long take_packet(unsigned long long *work,
 // every step instead of every pop cost 12 % there, and leaving after 64 pops instead
 // of 128 sent packets to the list that were about to end (nearest 11.23).
 constexpr int kDeferPops = 128;  // the batch's counter is read every so many pops
-struct DeferArgs
-{
-    uint4 *list = nullptr;      // (query, candidate's distance bits, rank or key, triangle or edge); nullptr: off
-    uint32_t *count = nullptr;  // entries reserved; may pass capacity, by entries that are not in the list
-    uint32_t capacity = 0;
-};
 // Whether the packet stops here: the lanes whose queries went to the list, 0 = it
 // goes on (the batch is not handed out yet, or the list is full). work: the
 // batch-wide packet counter, total: the batch's queries, lanes: those not yet
@@ -3262,6 +3294,14 @@ inline bool coop_ok(const TreeView &t, int packet, int width, int block, bool pe
     return t.near_first && packet == 2 && width == 2 && block == 128 && !persistent && !seed.cap && t.num_tris > 1 &&
            !t.order_count && !t.out_batch_order_enabled;
 }
+// Above kCoopDirect queries the lanes take the short searches first (one query per
+// lane, up to kLaneTurns expansions) and a second launch finishes the others, one per
+// warp: 20,480-triangle sphere with half its faces, silhouettes from its inside, direct /
+// with the lanes first (ms): 60,000 queries 0.62 / 0.54, 30,000 0.37 / 0.43; from its
+// surface, where every search is short, 0.30 / 0.13 and 0.16 / 0.12; 2M-triangle scene,
+// 98,000 queries 1.35 / 1.06. 16 / 64 / 128 expansions: walk on stars, 100,003 walkers,
+// 31.7 / 31.1 / 37.0 ms, 32 28.7.
+constexpr int64_t kCoopDirect = 24576;
 constexpr int64_t kCoopNearestMax = 98304, kCoopSilhouetteMax = 131072;
 // the wide searches serve near-first, one-thread-per-query, uncapped launches
 // over a tree whose wide records of that width exist
@@ -3347,6 +3387,34 @@ cudaError_t launch_deferring(void (*kernel)(KArgs...), int64_t n, cudaStream_t s
     {
         finish(d, 16 * sms);
         note_launch();
+        e = cudaGetLastError();
+    }
+    const cudaError_t f = cudaFreeAsync(scratch, st);
+    return e != cudaSuccess ? e : f;
+}
+// One query per lane, whose long ones end in a second launch: launch(d) and finish(d,
+// blocks) enqueue the two
+template <typename Launch, typename Finish>
+cudaError_t launch_lanes_deferring(int64_t n, cudaStream_t st, Launch launch, Finish finish)
+{
+    int dev = 0, sms = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess)
+        e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    char *scratch = nullptr;
+    if (e != cudaSuccess ||
+        (e = scratch_alloc_raw(reinterpret_cast<void **>(&scratch), 256 + 16 * (size_t)n, st)) != cudaSuccess)
+        return e;
+    DeferArgs d;
+    d.count = reinterpret_cast<uint32_t *>(scratch);
+    d.list = reinterpret_cast<uint4 *>(scratch + 256);
+    d.capacity = (uint32_t)n;
+    e = cudaMemsetAsync(scratch, 0, 8, st);
+    if (e == cudaSuccess)
+    {
+        launch(d);
+        finish(d, 16 * (unsigned)sms);
+        note_launch(2);
         e = cudaGetLastError();
     }
     const cudaError_t f = cudaFreeAsync(scratch, st);
@@ -3507,6 +3575,19 @@ cudaError_t launch_nearest(const TreeView &t0, const float *pts, int64_t n, uint
                         : launch_persistent(nearest_persistent_kernel<false>, n, st, t, pts, n, idx, dist, seed);
         launched = true;
     }
+    else if (coop && n > kCoopDirect)
+    {
+        e = launch_lanes_deferring(
+            n, st,
+            [&](const DeferArgs &d) {
+                nearest_fast_kernel<false, 128, true><<<grid_for(n, 128), 128, 0, st>>>(t, pts, n, idx, dist, nullptr,
+                                                                                       seed, d);
+            },
+            [&](const DeferArgs &d, unsigned blocks) {
+                nearest_finish_kernel<<<blocks, 32 * kCoopWarps, 0, st>>>(t, pts, idx, dist, seed, d);
+            });
+        launched = true;
+    }
     else if (coop)
         nearest_coop_kernel<<<grid_for(n, kCoopWarps), 32 * kCoopWarps, 0, st>>>(t, pts, n, idx, dist, seed);
     else if (t.near_first && t.block_near == 64)
@@ -3605,6 +3686,19 @@ cudaError_t launch_silhouette(const TreeView &t0, const float *pts, const uint8_
         e = seed.radius
                 ? launch_persistent(silhouette_persistent_kernel<true>, n, st, t, pts, flip, n, dist, edge, seed)
                 : launch_persistent(silhouette_persistent_kernel<false>, n, st, t, pts, flip, n, dist, edge, seed);
+        launched = true;
+    }
+    else if (coop && n > kCoopDirect)
+    {
+        e = launch_lanes_deferring(
+            n, st,
+            [&](const DeferArgs &d) {
+                silhouette_fast_kernel<false, 128, true>
+                    <<<grid_for(n, 128), 128, 0, st>>>(t, pts, flip, n, dist, edge, nullptr, seed, d);
+            },
+            [&](const DeferArgs &d, unsigned blocks) {
+                silhouette_finish_kernel<<<blocks, 32 * kCoopWarps, 0, st>>>(t, pts, flip, dist, edge, seed, d);
+            });
         launched = true;
     }
     else if (coop)

@@ -62,20 +62,22 @@ def test_small_batches(snch, level, n):
     same(*both_forms(snch, s, lambda: s.query_nearest(p) + s.query_silhouette(p, f)))
 
 
-# around the sizes where a batch is ordered (65,536), where nearest (98,304) and
+# around the sizes where the lanes take the short searches first (24,576), where a
+# batch is ordered (65,536), where nearest (98,304) and
 # silhouette (131,072) batches become packets, and where packets draw from the
 # per-SM pools (2^15 packets), closed mesh: packets of thousands of steps
-@pytest.mark.parametrize("n", [65_535, 65_536, 98_304, 98_305, 131_072, 131_073, 32 * 2**15 - 31, 32 * 2**15 + 1])
+@pytest.mark.parametrize("n", [24_576, 24_577, 65_535, 65_536, 98_304, 98_305, 131_072, 131_073, 32 * 2**15 - 31, 32 * 2**15 + 1])
 def test_size_rules_on_a_closed_mesh(snch, n):
     s = scene(snch, 5)
     p, f = points(n, seed=7)
     same(*both_forms(snch, s, lambda: s.query_nearest(p) + s.query_silhouette(p, f)))
 
 
-def test_seeded_small_batches(snch):
+@pytest.mark.parametrize("n", [5000, 30_000])
+def test_seeded_small_batches(snch, n):
     import torch
     s = scene(snch, 4)
-    p, f = points(5000, seed=3)
+    p, f = points(n, seed=3)
     i, d = s.query_nearest(p)
     sd, e = s.query_silhouette(p, f)
     for scale in (0.5, 1.0, 2.0):  # below, at and above the answers
@@ -86,7 +88,7 @@ def test_seeded_small_batches(snch):
         same(b, (i, d, sd, e))
 
 
-@pytest.mark.parametrize("n", [777, 200_000])
+@pytest.mark.parametrize("n", [777, 30_001, 200_000])
 def test_batched_scene(snch, n):
     import torch
     meshes = [mesh(k) for k in (-1, 3, 5, -2)] + [(np.zeros((0, 3), np.float32), np.zeros((0, 3), np.int32))]
