@@ -18,11 +18,11 @@
 // table is laid out along the vertices: an edge starts at one of the places of its
 // smaller vertex, so neighbouring triangles, which share vertices, work on
 // neighbouring sectors that stay in L2 (most meshes number their vertices along
-// their surface). A start that is taken kLocalProbes times over goes on from a hash of
-// the whole key: a vertex with a million edges costs a few more probes, no more.
+// their surface). After kLocalProbes taken places the probes jump by hashes of the whole
+// key: a vertex with a million edges costs a few more probes (1M triangles 0.45 ms).
 // One table each for keys, first and last occurrences, by a hash of the key: 2M
 // triangles, insert + flags + scan + finalise 410 + 40 + 60 + 264 us, bound by random
-// sectors, against 152 + 44 + 9 + 68 us (and a smaller table to clear) here.
+// sectors, against 160 + 44 + 9 + 68 us (and a smaller table to clear) here.
 #include "common.cuh"
 #include "internal.h"
 
@@ -32,7 +32,7 @@ namespace
 {
 
 constexpr unsigned long long kEmpty = ~0ull;
-constexpr uint32_t kLocalProbes = 8;
+constexpr uint32_t kLocalProbes = 4, kJumps = 64;
 
 // all bits set = empty; last occurrences as kInvalid - (k + 1), so that every field's
 // reduction is a minimum from the same initial value (kInvalid: none)
@@ -67,22 +67,34 @@ __device__ __forceinline__ unsigned long long mix64(unsigned long long k)
     return k;
 }
 
-// the slot of the edge (found or claimed), kInvalid if the table is full
+// the slot of the edge (found or claimed), kInvalid if the table is full. Places of
+// consecutive vertices with many edges each fill up into runs of thousands of full
+// slots, so the probes after the local ones jump (a walk along such a run took 0.7 ms
+// for a sphere of 10,000 triangles); at two thirds full, 64 jumps all fail once in 1e11,
+// and the walk over the whole table after them only makes the search complete.
 __device__ __forceinline__ uint32_t find_or_claim(const Table &t, uint32_t lo, uint32_t hi)
 {
-    const unsigned long long key = ((unsigned long long)lo << 32) | hi, h64 = mix64(key);
-    const uint32_t far = (uint32_t)(((h64 >> 32) * t.cap) >> 32);
-    uint32_t h = far;
-    if (t.stride)
-        h = lo * t.stride + (uint32_t)((h64 & 0xFFFFFFFFull) * t.stride >> 32);
-    for (uint64_t probe = 0; probe < kLocalProbes + (uint64_t)t.cap; ++probe)
+    const unsigned long long key = ((unsigned long long)lo << 32) | hi;
+    unsigned long long h64 = mix64(key);
+    uint32_t h = t.stride ? lo * t.stride + (uint32_t)((h64 & 0xFFFFFFFFull) * t.stride >> 32)
+                          : (uint32_t)(((h64 >> 32) * t.cap) >> 32);
+    for (uint64_t probe = 0; probe < kLocalProbes + kJumps + (uint64_t)t.cap; ++probe)
     {
-        if (probe == kLocalProbes && t.stride)
-            h = far;
-        const unsigned long long prev = atomicCAS(&t.slots[h].key, kEmpty, key);
+        // a key never changes once set, so a cached read may only be late, seeing the
+        // slot still empty; other keys are passed without an atomic (a fan of 1M
+        // triangles queued 10 ms on its centre's few slots)
+        unsigned long long prev = *reinterpret_cast<const unsigned long long *>(&t.slots[h].key);
+        if (prev == kEmpty)
+            prev = atomicCAS(&t.slots[h].key, kEmpty, key);
         if (prev == kEmpty || prev == key)
             return h;
-        h = h + 1 < t.cap ? h + 1 : 0;
+        if (probe + 1 >= kLocalProbes && probe + 1 < kLocalProbes + kJumps)
+        {
+            h64 = mix64(h64 + 0x9E3779B97F4A7C15ull);
+            h = (uint32_t)(((h64 >> 32) * t.cap) >> 32);
+        }
+        else
+            h = h + 1 < t.cap ? h + 1 : 0;
     }
     return kInvalid;
 }
@@ -282,6 +294,12 @@ inline Layout layout(uint32_t num_tris)
     l.before = l.counts + words;
     l.scan = l.before + words;
     l.total = l.scan + al(scan_flags_scratch_bytes(flag_words(num_tris)));
+    // up to a quarter of a power of two, so that scenes of about the same size share
+    // cached blocks
+    size_t step = 256;
+    while (8 * step <= l.total)
+        step <<= 1;
+    l.total = (l.total + step - 1) / step * step;
     return l;
 }
 

@@ -43,6 +43,14 @@ def soup(n, rng):
     return v.astype(np.float32), np.arange(3 * n).reshape(n, 3).astype(np.int32)
 
 
+def two_levels(n, rng):
+    """Edges that all have their smaller vertex among the first few (an icosphere's coarse
+    vertices come first), half of the triangles missing: those vertices' places overflow."""
+    from snch_lbvh_gb300 import meshes
+    v, f, _ = meshes.icosphere(4)
+    return v.astype(np.float32), f[rng.permutation(len(f))[:n]]
+
+
 def sparse(n, rng):
     """A height field whose vertices are spread over many unused ones."""
     v, f = grid(n, rng)
@@ -67,7 +75,7 @@ def device_words(ptr, rows, words):
 
 
 CASES = [(grid, n) for n in (1, 2, 3, 255, 256, 257, 511, 512, 513, 1365, 1366, 43_691, 100_000)] + \
-        [(fan, 5000), (soup, 3000), (sparse, 700), (degenerate, 900)]
+        [(fan, 5000), (fan, 200_000), (soup, 3000), (two_levels, 2560), (sparse, 700), (degenerate, 900)]
 
 
 @pytest.mark.parametrize("make,n", CASES, ids=[f"{m.__name__}-{n}" for m, n in CASES])
