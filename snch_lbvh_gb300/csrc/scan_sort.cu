@@ -151,14 +151,31 @@ __global__ void radix_hist_kernel(const uint32_t *__restrict__ keys, uint32_t n,
     }
 }
 
+// the lanes of `among` with this lane's digit, a ballot per bit: a one-instruction
+// __match_any_sync is slower (16M pairs, one pass: 156 us, against 128 here)
+__device__ __forceinline__ uint32_t same_digit(uint32_t d, uint32_t among)
+{
+    uint32_t peers = among;
+#pragma unroll
+    for (int b = 0; b < 8; ++b)
+    {
+        const bool bit = (d >> b) & 1u;
+        const uint32_t m = __ballot_sync(0xffffffffu, bit);
+        peers &= bit ? m : ~m;
+    }
+    return peers;
+}
+
 // One 8-bit digit pass. Warp w ranks elements [tile*4096 + w*512, +512) in 16
-// rounds of 32 with __match_any_sync, which keeps equal digits in input order;
+// rounds of 32 by same_digit, which keeps equal digits in input order;
 // the block then stages the tile in shared memory in digit order and writes
 // each digit run to its global position.
-// (The compiler's 80 registers allow 3 blocks per SM. Compiled for 4 or 5 blocks,
-// with the largest shared-memory carveout so that the 42 KB of shared memory
-// per block fit, the 16M-pair sort took 0.576 / 0.586 against 0.570 ms.)
-__global__ void __launch_bounds__(kThreads) onesweep_pass_kernel(
+// Bound by the latency of a tile (ranking, staging, look-back), so by the tiles in
+// flight: 3 blocks per SM, 80 registers. Left to itself the compiler takes 128 registers
+// and 2 blocks (174 us a pass of 16M pairs); for 4 / 5 blocks it spills (155 / 132 us).
+// Requesting 4, 8 or 16 earlier tiles' states at once in the look-back was slower (167 to
+// 172 against 156 us before): a tile waits for its neighbours to publish, not for reads.
+__global__ void __launch_bounds__(kThreads, 3) onesweep_pass_kernel(
     const uint32_t *__restrict__ keys_in, const uint32_t *__restrict__ vals_in, uint32_t *__restrict__ keys_out,
     uint32_t *__restrict__ vals_out, uint32_t n, int shift, const uint32_t *__restrict__ hist, uint32_t *lookback,
     uint32_t *tile_counter, uint32_t *status)
@@ -190,15 +207,18 @@ __global__ void __launch_bounds__(kThreads) onesweep_pass_kernel(
         v[r] = ok ? vals_in[e] : 0u;
     }
     const uint32_t lt = (1u << lane) - 1u;
+    const bool full = (uint64_t)(tile + 1) * kSortTile <= n;
 #pragma unroll
     for (int r = 0; r < kRounds; ++r)
     {
         const uint64_t e = base + r * 32 + lane;
-        const uint32_t d = (e < n) ? ((k[r] >> shift) & 255u) : 256u;
-        const uint32_t peers = __match_any_sync(0xffffffffu, d);
+        const uint32_t d = (k[r] >> shift) & 255u;
+        // lanes past the end (the last tile's) keep out of the valid lanes' counts
+        const uint32_t in = full ? 0xffffffffu : __ballot_sync(0xffffffffu, e < n);
+        const uint32_t peers = same_digit(d, (in >> lane) & 1u ? in : ~in);
         const int leader = __ffs(peers) - 1;
         uint32_t cnt = 0;
-        if (lane == leader && d < 256u)
+        if (lane == leader && ((in >> lane) & 1u))
         {
             cnt = s_warp_hist[warp][d];
             s_warp_hist[warp][d] = cnt + __popc(peers);
