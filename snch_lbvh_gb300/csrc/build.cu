@@ -842,10 +842,8 @@ __global__ void __launch_bounds__(kRefitLeaves, 6) refit_kernel(BuildArgs a)
                 put_box(B + s, m);
                 a.aabbs[p] = m;
                 InnerRec ir = pack_inner(lb, rb, rec.y, rec.z);
-                if (rec.y >= ni)
-                    ir.d.z = __uint_as_float(s_info[rec.y - ni - b0]);
-                if (rec.z >= ni)
-                    ir.d.w = __uint_as_float(s_info[rec.z - ni - b0]);
+                ir.d.z = __uint_as_float(rec.y >= ni ? s_info[rec.y - ni - b0] : cone_info(get_cone(slot_of(rec.y))));
+                ir.d.w = __uint_as_float(rec.z >= ni ? s_info[rec.z - ni - b0] : cone_info(get_cone(slot_of(rec.z))));
                 a.inner[p] = ir;
             }
             const Cone lc = get_cone(slot_of(rec.y)), rc = get_cone(slot_of(rec.z));
@@ -901,10 +899,8 @@ __global__ void __launch_bounds__(128) refit_top_kernel(BuildArgs a)
             const f3 cm = centroid(m);
             a.cones[p] = cone_merge(lc, rc, sqlen3(sub(cm, centroid(lb))), sqlen3(sub(cm, centroid(rb))));
             InnerRec ir = pack_inner(lb, rb, L, R);
-            if (L >= ni)
-                ir.d.z = __uint_as_float(scratch.info[L - ni]);
-            if (R >= ni)
-                ir.d.w = __uint_as_float(scratch.info[R - ni]);
+            ir.d.z = __uint_as_float(L >= ni ? scratch.info[L - ni] : cone_info(lc));
+            ir.d.w = __uint_as_float(R >= ni ? scratch.info[R - ni] : cone_info(rc));
             a.inner[p] = ir;
             a.inner_cones[p] = pack_cones(lc, rc);
             up = p;

@@ -59,15 +59,18 @@ struct NodeRec
 // boxes and both child node ids, so expanding a node is one 64-B line
 // (four 16-B vector loads) instead of the reference's four scattered records.
 //   a = (L.upper.xyz, L.lower.x)  b = (L.lower.yz, R.upper.xy)
-//   c = (R.upper.z, R.lower.xyz)  d = (bits L, bits R, 0, 0)
+//   c = (R.upper.z, R.lower.xyz)  d = (bits L, bits R, info L, info R)
 // d = (bits L, bits R, leaf info of L, leaf info of R); a leaf child's info is
-// its DFS rank | owned-edge count << 30 (written by the rank pass), so the
-// silhouette traversal reaches a leaf's edges without reading its LeafRec.
+// its DFS rank | owned-edge count << 30, so the silhouette traversal reaches a leaf's
+// edges without reading its LeafRec; an internal child's says whether its cone test is
+// settled whatever the query (kConePass: half angle of 90 degrees or more, kConeFail: no
+// edges), so that a node whose children are both settled is expanded without its cones.
 struct alignas(64) InnerRec
 {
     float4 a, b, c, d;
 };
 constexpr uint32_t kLeafRankMask = (1u << 30) - 1u;
+constexpr uint32_t kConePass = 1u, kConeFail = 2u;  // 0: depends on the query (or an older file)
 // Child cones of an internal node (silhouette traversal), 48 B:
 //   a = (L.axis.xyz, L.half)  b = (L.radius, R.axis.xyz)  c = (R.half, R.radius, 0, 0)
 struct alignas(16) InnerConeRec
@@ -357,6 +360,11 @@ SNCH_DEV void unpack_cones(const InnerConeRec &r, Cone &l, Cone &rc)
     rc.axis = mk(r.b.y, r.b.z, r.b.w);
     rc.half_angle = r.c.x;
     rc.radius = r.c.y;
+}
+// InnerRec info of an internal child with this cone
+SNCH_DEV uint32_t cone_info(const Cone &c)
+{
+    return c.half_angle >= kPi2 ? kConePass : c.half_angle < 0.0f ? kConeFail : 0u;
 }
 SNCH_DEV InnerConeRec pack_cones(const Cone &l, const Cone &r)
 {

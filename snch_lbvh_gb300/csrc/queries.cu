@@ -1939,23 +1939,35 @@ SNCH_DEV void silhouette_packet_chunk(const TreeView &t, const float *__restrict
             {
                 if (kStats)
                     ++n_int;
-                InnerConeRec icr;
-                if (in_top)
-                    icr = s_topc[slot];
-                else
-                {
-                    const float4 *cr = reinterpret_cast<const float4 *>(t.inner_cones + node);
-                    icr.a = __ldg(cr);
-                    icr.b = __ldg(cr + 1);
-                    icr.c = __ldg(cr + 2);
-                }
-                Cone lc, rc;
-                unpack_cones(icr, lc, rc);
                 Lmd = mindist(lb, p);
                 Rmd = mindist(rb, p);
                 const float b2 = best * best;
-                hitL = Lmd <= b2 && lc.half_angle >= 0.0f && cone_test(lc, p, lb, Lmd);
-                hitR = Rmd <= b2 && rc.half_angle >= 0.0f && cone_test(rc, p, rb, Rmd);
+                hitL = Lmd <= b2;
+                hitR = Rmd <= b2;
+                if (L < ni && R < ni && Linfo != 0u && Rinfo != 0u)
+                {
+                    // both cone tests are settled: no cone record is read (a uniform
+                    // branch; 16M queries of the 2M-triangle scene 32.3 -> 31.5 ms)
+                    hitL = hitL && Linfo == kConePass;
+                    hitR = hitR && Rinfo == kConePass;
+                }
+                else
+                {
+                    InnerConeRec icr;
+                    if (in_top)
+                        icr = s_topc[slot];
+                    else
+                    {
+                        const float4 *cr = reinterpret_cast<const float4 *>(t.inner_cones + node);
+                        icr.a = __ldg(cr);
+                        icr.b = __ldg(cr + 1);
+                        icr.c = __ldg(cr + 2);
+                    }
+                    Cone lc, rc;
+                    unpack_cones(icr, lc, rc);
+                    hitL = hitL && lc.half_angle >= 0.0f && cone_test(lc, p, lb, Lmd);
+                    hitR = hitR && rc.half_angle >= 0.0f && cone_test(rc, p, rb, Rmd);
+                }
                 // the leaf work of both children as one loop of edge_candidate calls
                 // (the left leaf's edges, then the right leaf's, per lane: the order of
                 // two leaf_silhouette_info calls), so a lane with only the right leaf

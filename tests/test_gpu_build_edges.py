@@ -98,7 +98,8 @@ def test_topology_and_tree(snch, oracle_mod, make, n):
         check_cones(t["cones"], orc.cones, orc.nodes, orc.d1)
         np.testing.assert_array_equal(s.leaf_ranks(), orc.leaf_ranks())
     assert s.device_status() == 0
-    # the traversal records: child ids, and rank and owned-edge count of leaf children
+    # the traversal records: child ids, rank and owned-edge count of leaf children, and
+    # whether an internal child's cone test is settled
     if n > 1:
         t_ = len(f)
         rec = device_words(s.get_traversal_view().inner, t_ - 1, 16).view(np.uint32)
@@ -106,7 +107,9 @@ def test_topology_and_tree(snch, oracle_mod, make, n):
         owned = (orc.tri_owned[orc.sorted_idx] >= 0).sum(1).astype(np.uint32)
         info = (orc.leaf_ranks() | owned << 30).astype(np.uint32)
         child = rec[:, 12:14].astype(np.int64) - (t_ - 1)
-        np.testing.assert_array_equal(rec[:, 14:16], np.where(child >= 0, info[child.clip(0)], 0))
+        half = t["cones"][orc.nodes[: t_ - 1, 1:3], 3]  # the built tree's own half angles
+        settled = np.where(half >= np.float32(np.pi / 2), 1, np.where(half < 0, 2, 0))
+        np.testing.assert_array_equal(rec[:, 14:16], np.where(child >= 0, info[child.clip(0)], settled))
         np.testing.assert_array_equal(rec[:, :12], bits(orc.aabbs)[orc.nodes[: t_ - 1, 1:3]].reshape(-1, 12))
     # near-first against the reference's order (ids up to the documented exact ties)
     p = torch.from_numpy((rng.random((2000, 3)) * (v.max(0) - v.min(0) + 0.1) + v.min(0)).astype(np.float32)).cuda()
