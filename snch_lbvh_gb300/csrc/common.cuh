@@ -342,14 +342,21 @@ SNCH_DEV InnerRec pack_inner(const Box &l, const Box &r, uint32_t L, uint32_t R)
     o.d = make_float4(__uint_as_float(L), __uint_as_float(R), 0.0f, 0.0f);
     return o;
 }
+// 32 bytes in one load (ld.global.nc.v8, sm_100 and later), p 32-byte aligned: half the
+// loads of a 64-byte record (records are 64-byte aligned, their arrays 256). Against
+// 16-byte loads (ms): 24 batched meshes 36.2 -> 33.5, 4M sphere draws 0.815 -> 0.78, 16M
+// rays 7.87 -> 7.72, nearest 10.16 -> 10.04, silhouettes 31.4 -> 31.2.
+SNCH_DEV void load32(const void *p, float4 &a, float4 &b)
+{
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+        : "l"(p));
+}
 SNCH_DEV InnerRec load_inner(const InnerRec *p)
 {
-    const float4 *q = reinterpret_cast<const float4 *>(p);
     InnerRec r;
-    r.a = __ldg(q);
-    r.b = __ldg(q + 1);
-    r.c = __ldg(q + 2);
-    r.d = __ldg(q + 3);
+    load32(p, r.a, r.b);
+    load32(&p->c, r.c, r.d);
     return r;
 }
 SNCH_DEV void unpack_cones(const InnerConeRec &r, Cone &l, Cone &rc)

@@ -813,7 +813,8 @@ SNCH_DEV void edge_record_candidate(const TreeView &t, uint64_t slot, uint32_t k
                                     uint32_t &best_key, int32_t &best_edge)
 {
     const float4 *e = reinterpret_cast<const float4 *>(t.edges + slot);
-    const float4 ea = __ldg(e), eb = __ldg(e + 1);
+    float4 ea, eb;
+    load32(e, ea, eb);
     const f3 pa = mk(ea.x, ea.y, ea.z), pb = mk(eb.x, eb.y, eb.z);
     f3 cp;
     const float sq = closest_point_segment_sq(pa, pb, o, cp);
@@ -826,7 +827,8 @@ SNCH_DEV void edge_record_candidate(const TreeView &t, uint64_t slot, uint32_t k
     bool is_sil = (flags & 1u) == 0u || (flags & 2u) == 0u;
     if (!is_sil)
     {
-        const float4 ec = __ldg(e + 2), ed = __ldg(e + 3);
+        float4 ec, ed;
+        load32(e + 2, ec, ed);
         is_sil = is_silhouette_edge(pa, pb, mk(ec.x, ec.y, ec.z), mk(ed.x, ed.y, ed.z),
                                     mk(o.x - cp.x, o.y - cp.y, o.z - cp.z), d, flip);
     }
