@@ -2954,8 +2954,24 @@ __global__ void __launch_bounds__(128) sample_kernel(TreeView t, const float *__
             unpack_inner(load_inner(t.inner + node), lb, rb, L, R);
             if (kStats)
                 ++n_int;
-            const float Lw = sphere_box(c, rad, lb) ? green_weight(c, centroid(lb)) : 0;
-            const float Rw = sphere_box(c, rad, rb) ? green_weight(c, centroid(rb)) : 0;
+            // One child only: its share is weight / weight, 1, and the draw goes there with u
+            // and the density unchanged (u / 1, 1 * density), so the weights (a square root
+            // and a division each) and the two divisions of the choice are not computed.
+            // A weight is 0, which ends the draw, only if the squared distance overflows;
+            // u outside [0, 1), after rounding or by the caller, takes the general form.
+            const bool Lh = sphere_box(c, rad, lb), Rh = sphere_box(c, rad, rb);
+            if (!(Lh || Rh))
+                break;
+            if (Lh != Rh && u >= 0.0f && u < 1.0f)
+            {
+                const f3 m = centroid(Lh ? lb : rb);
+                if (sqlen3(mk(c.x - m.x, c.y - m.y, c.z - m.z)) == INFINITY)
+                    break;
+                node = Lh ? L : R;
+                continue;
+            }
+            const float Lw = Lh ? green_weight(c, centroid(lb)) : 0;
+            const float Rw = Rh ? green_weight(c, centroid(rb)) : 0;
             const float tw = Lw + Rw;
             if (!(tw > 0))
                 break;
