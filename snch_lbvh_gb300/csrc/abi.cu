@@ -1051,9 +1051,20 @@ int snch_build_bvh(snch_scene_t s, snch_stream_t stream)
     if (s->num_tris > 0)
     {
         BuildArgs a = build_args(s);
-        SNCH_CUDA(launch_build_front(a, st));
-        SNCH_CUDA(radix_sort_pairs(s->keys, s->vals, s->keys_tmp, s->vals_tmp, s->num_tris, 30, s->small + kWHist,
-                                   s->scratch, s->small + kWStatus, st));
+        if (s->num_tris <= kRankSortMax)
+        {
+            BuildArgs front = a;
+            front.keys = s->keys_tmp;
+            front.vals = s->vals_tmp;
+            SNCH_CUDA(launch_build_front(front, st));
+            SNCH_CUDA(rank_sort_pairs(s->keys_tmp, s->vals_tmp, s->keys, s->vals, s->num_tris, st));
+        }
+        else
+        {
+            SNCH_CUDA(launch_build_front(a, st));
+            SNCH_CUDA(radix_sort_pairs(s->keys, s->vals, s->keys_tmp, s->vals_tmp, s->num_tris, 30, s->small + kWHist,
+                                       s->scratch, s->small + kWStatus, st));
+        }
         SNCH_CUDA(launch_mesh_pass(a, s->scratch, st));  // batched scenes only
         SNCH_CUDA(launch_build_back(a, st));
         if (s->num_meshes == 0)

@@ -212,6 +212,13 @@ struct SortResult
 cudaError_t radix_sort_pairs(uint32_t *keys, uint32_t *vals, uint32_t *keys_tmp, uint32_t *vals_tmp, uint32_t n,
                              int key_bits, const uint32_t *hist, void *scratch, uint32_t *status, cudaStream_t st,
                              SortResult *result = nullptr);
+// Small arrays in one launch (rank_sort_kernel): the stable order of the whole keys, from
+// (keys_in, vals_in) to (keys_out, vals_out), which must not overlap. Its work grows with
+// n^2: tree build of n triangles, radix passes / ranks, us: 306 103 / 70, 1,260 113 / 83,
+// 5,112 136 / 104, 11,990 144 / 124, 15,876 143 / 140, 20,306 147 / 164.
+constexpr uint32_t kRankSortMax = 12288;
+cudaError_t rank_sort_pairs(const uint32_t *keys_in, const uint32_t *vals_in, uint32_t *keys_out, uint32_t *vals_out,
+                            uint32_t n, cudaStream_t st);
 inline int sort_passes(int key_bits) { return (key_bits + 7) / 8; }
 
 // ---- topology.cu (scene.cuh:1135-1225 on the device)

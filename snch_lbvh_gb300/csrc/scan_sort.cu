@@ -283,6 +283,75 @@ __global__ void __launch_bounds__(kThreads, 3) onesweep_pass_kernel(
 
 inline uint32_t num_tiles(uint64_t n) { return (uint32_t)((n + kSortTile - 1) / kSortTile); }
 
+// Small sorts by rank: a pair's place is the number of pairs before it (smaller key, or
+// the same key and earlier), counted against every other pair. The radix passes of a small
+// array are a chain of launches with a few blocks each (clear, histogram and four passes:
+// about 40 us); this is one. A lane counts for one key, the block's warps share the other
+// keys, 128 at a time through shared memory, read back four to a broadcast. Bound by the
+// comparisons, two instructions each.
+constexpr int kRankWarps = 8, kRankChunk = 128;
+__global__ void __launch_bounds__(32 * kRankWarps) rank_sort_kernel(const uint32_t *__restrict__ keys_in,
+                                                                    const uint32_t *__restrict__ vals_in,
+                                                                    uint32_t *__restrict__ keys_out,
+                                                                    uint32_t *__restrict__ vals_out, uint32_t n)
+{
+    __shared__ uint4 s_keys[kRankWarps][kRankChunk / 4];
+    __shared__ uint32_t s_before[kRankWarps][32];
+    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const uint32_t i = blockIdx.x * 32u + lane;
+    const uint32_t key = i < n ? __ldg(keys_in + i) : 0u;
+    const uint32_t own = blockIdx.x * 32u / kRankChunk;  // the chunk that holds this block's keys
+    const uint32_t chunks = (n + kRankChunk - 1) / kRankChunk;
+    uint32_t *mine = reinterpret_cast<uint32_t *>(s_keys[w]);
+    uint32_t before = 0;
+    for (uint32_t c = w; c < chunks; c += kRankWarps)
+    {
+        __syncwarp();
+#pragma unroll
+        for (uint32_t k = 0; k < kRankChunk; k += 32)
+        {
+            const uint32_t j = c * kRankChunk + k + lane;
+            mine[k + lane] = j < n ? __ldg(keys_in + j) : 0xffffffffu;  // no key is above it
+        }
+        __syncwarp();
+        if (c < own)  // earlier pairs: equal keys count
+        {
+#pragma unroll 8
+            for (int k = 0; k < kRankChunk / 4; ++k)
+            {
+                const uint4 v = s_keys[w][k];
+                before += (uint32_t)(v.x <= key) + (uint32_t)(v.y <= key) + (uint32_t)(v.z <= key) +
+                          (uint32_t)(v.w <= key);
+            }
+        }
+        else if (c > own)
+        {
+#pragma unroll 8
+            for (int k = 0; k < kRankChunk / 4; ++k)
+            {
+                const uint4 v = s_keys[w][k];
+                before += (uint32_t)(v.x < key) + (uint32_t)(v.y < key) + (uint32_t)(v.z < key) + (uint32_t)(v.w < key);
+            }
+        }
+        else
+            for (uint32_t k = 0; k < kRankChunk; ++k)
+            {
+                const uint32_t v = mine[k];
+                before += (uint32_t)(v < key || (v == key && c * kRankChunk + k < i));
+            }
+    }
+    s_before[w][lane] = before;
+    __syncthreads();
+    if (w != 0 || i >= n)
+        return;
+    uint32_t at = 0;
+#pragma unroll
+    for (int k = 0; k < kRankWarps; ++k)
+        at += s_before[k][lane];
+    keys_out[at] = key;
+    vals_out[at] = __ldg(vals_in + i);
+}
+
 }  // namespace
 
 size_t scan_flags_scratch_bytes(uint64_t n) { return 4 * (size_t)(num_tiles(n) + 1); }
@@ -299,6 +368,16 @@ cudaError_t scan_flags(const uint32_t *in, uint32_t *out, uint32_t n, uint32_t *
     if (e != cudaSuccess)
         return e;
     scan_flags_kernel<<<tiles, kThreads, 0, st>>>(in, out, n, total, state, counter, status);
+    note_launch();
+    return cudaGetLastError();
+}
+
+cudaError_t rank_sort_pairs(const uint32_t *keys_in, const uint32_t *vals_in, uint32_t *keys_out, uint32_t *vals_out,
+                            uint32_t n, cudaStream_t st)
+{
+    if (n == 0)
+        return cudaSuccess;
+    rank_sort_kernel<<<(n + 31) / 32, 32 * kRankWarps, 0, st>>>(keys_in, vals_in, keys_out, vals_out, n);
     note_launch();
     return cudaGetLastError();
 }

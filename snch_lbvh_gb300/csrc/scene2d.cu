@@ -1219,11 +1219,22 @@ int snch_scene2_build(snch_scene2_t s, snch_stream_t stream)
                  s->leaf_verts};
         init2_kernel<<<1, 32, 0, st>>>(s->small);
         leaf2_kernel<<<blocks(n, 256), 256, 0, st>>>(a);
+        const bool ranks = n <= kRankSortMax;
+        if (ranks)
+        {
+            a.keys = s->keys_tmp;
+            a.vals = s->vals_tmp;
+        }
         morton2_kernel<<<blocks(n, 256), 256, 0, st>>>(a);
         note_launch(3);
         SNCH2_CUDA(cudaGetLastError());
-        SNCH2_CUDA(radix_sort_pairs(s->keys, s->vals, s->keys_tmp, s->vals_tmp, n, 30, nullptr, s->scratch,
-                                    s->small + 8, st));
+        if (ranks)
+            SNCH2_CUDA(rank_sort_pairs(a.keys, a.vals, s->keys, s->vals, n, st));
+        else
+            SNCH2_CUDA(radix_sort_pairs(s->keys, s->vals, s->keys_tmp, s->vals_tmp, n, 30, nullptr, s->scratch,
+                                        s->small + 8, st));
+        a.keys = s->keys;
+        a.vals = s->vals;
         BuildArgs k{};
         k.num_tris = n;
         k.keys = s->keys;
