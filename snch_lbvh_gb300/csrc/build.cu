@@ -4,7 +4,8 @@
 //                       block-reduced scene AABB (bvh.cuh:428-432) via ordered atomics
 //   morton_kernel       30-bit codes (bvh.cuh:292-302, morton_code.cuh:19-70) and the
 //                       digit histograms of all four radix passes in the same read
-//   [radix_sort_pairs]  stable onesweep sort of (code, triangle index), scan_sort.cu
+//   [radix_sort_pairs]  stable onesweep sort of (code, triangle index), scan_sort.cu; small
+//                       builds: rank_sort_pairs, one launch
 //   karras_kernel       internal nodes (bvh.cuh:109-229) with the reference's node
 //                       numbering; ties of equal codes broken by the sorted object
 //                       index exactly as the 64-bit (code << 32 | idx) keys do
@@ -628,7 +629,7 @@ SNCH_DEV Cone ldcg_cone(const Cone *p)
 // One walk per leaf from its records to the root through global memory, in one kernel,
 // took 864 us for 2M triangles and the ranks 85 us in another: the walk holds its
 // block's place while one lane of it waits for fences, an atomic and three dependent
-// reads a level, and the gathers of the leaves wait for few warps. Here 250 + 204 + 74
+// reads a level, and the gathers of the leaves wait for few warps. Here 250 + 204 + 66
 // us (one kernel for all three: 770 us, held up by the walks at its end).
 constexpr int kRefitLeaves = 256;
 
@@ -874,7 +875,10 @@ SNCH_DEV uint32_t arrive_acq_rel(uint32_t *p)
     return old;
 }
 // The first thread to reach a node stops; the second (whose sibling's results are
-// published by the sibling's arrival, or by the end of refit_kernel) merges.
+// published by the sibling's arrival, or by the end of refit_kernel) merges. Bound by the
+// chain of arrivals and merges, so a thread carries its own node's box and cone up and asks
+// for the parent's record before it arrives (2M triangles 72 -> 66 us; reading all of it
+// after the arrival costs two more round trips a level).
 __global__ void __launch_bounds__(128) refit_top_kernel(BuildArgs a)
 {
     const uint32_t ni = a.num_tris - 1;
@@ -883,27 +887,32 @@ __global__ void __launch_bounds__(128) refit_top_kernel(BuildArgs a)
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x)
     {
         uint32_t up = scratch.exits[i];
+        uint32_t p = __ldg(&a.nodes[up].parent);
+        Box box = ldcg_box(a.aabbs + up);
+        Cone cone = ldcg_cone(a.cones + up);
         // a Karras tree over 64-bit keys is at most 65 levels deep
-        for (int level = 0; level < 96; ++level)
+        for (int level = 0; level < 96 && p < ni; ++level)
         {
-            const uint32_t p = a.nodes[up].parent;
-            if (p >= ni)
-                break;
+            const uint4 rec = __ldg(reinterpret_cast<const uint4 *>(a.nodes + p));  // parent, left, right, object
             if (arrive_acq_rel(a.flags + p) == 0u)
                 break;
-            const uint32_t L = a.nodes[p].left, R = a.nodes[p].right;
-            const Box lb = ldcg_box(a.aabbs + L), rb = ldcg_box(a.aabbs + R);
-            const Cone lc = ldcg_cone(a.cones + L), rc = ldcg_cone(a.cones + R);
-            const Box m = merge_box(lb, rb);
-            a.aabbs[p] = m;
-            const f3 cm = centroid(m);
-            a.cones[p] = cone_merge(lc, rc, sqlen3(sub(cm, centroid(lb))), sqlen3(sub(cm, centroid(rb))));
+            const uint32_t L = rec.y, R = rec.z, other = L == up ? R : L;
+            const Box ob = ldcg_box(a.aabbs + other);
+            const Cone oc = ldcg_cone(a.cones + other);
+            const Box lb = L == up ? box : ob, rb = L == up ? ob : box;
+            const Cone lc = L == up ? cone : oc, rc = L == up ? oc : cone;
+            box = merge_box(lb, rb);
+            a.aabbs[p] = box;
+            const f3 cm = centroid(box);
+            cone = cone_merge(lc, rc, sqlen3(sub(cm, centroid(lb))), sqlen3(sub(cm, centroid(rb))));
+            a.cones[p] = cone;
             InnerRec ir = pack_inner(lb, rb, L, R);
             ir.d.z = __uint_as_float(L >= ni ? scratch.info[L - ni] : cone_info(lc));
             ir.d.w = __uint_as_float(R >= ni ? scratch.info[R - ni] : cone_info(rc));
             a.inner[p] = ir;
             a.inner_cones[p] = pack_cones(lc, rc);
             up = p;
+            p = rec.x;
         }
     }
 }
