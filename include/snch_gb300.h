@@ -321,8 +321,9 @@ int snch_set_traversal(snch_scene_t scene, int mode);
  *                             batch: 12 to 30, default 24 (a 256^3 grid, sorted in three
  *                             radix passes; measured on 16M-query batches of the
  *                             2M-triangle scene: 0.4 % faster per step than 30 bits in four
- *                             passes, 16 bits 52 % slower). Queries of one cell keep their
- *                             input order; only the speed changes. */
+ *                             passes, 16 bits 52 % slower). Batches of up to 2^17 points
+ *                             or 2^22 rays take 16 at most (two passes). Queries of one
+ *                             cell keep their input order; only the speed changes. */
 #define SNCH_OPT_ORDER_BITS 23
 /*   SNCH_OPT_HOST_CHUNK       queries per chunk of the *_host forms (at most 29 bytes in
  *                             and 17 out per query on each of two streams): chunk i's

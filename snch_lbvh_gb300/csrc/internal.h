@@ -202,9 +202,11 @@ cudaError_t scan_flags(const uint32_t *in, uint32_t *out, uint32_t n, uint32_t *
 // receives the buffer pair that holds it ((keys, vals) or (keys_tmp,
 // vals_tmp), after an odd number of passes) and nothing is copied back. If
 // hist is non-null it already holds the per-pass digit counts (passes x 256)
-// and the histogram pass is skipped.
+// and the histogram pass is skipped; hist == scratch: the counts were added up at the
+// start of the scratch after clear_sort_scratch.
 constexpr int kSortTile = 4096;
 size_t sort_scratch_bytes(uint32_t n, int key_bits);
+cudaError_t clear_sort_scratch(void *scratch, uint32_t n, int key_bits, cudaStream_t st);
 struct SortResult
 {
     uint32_t *keys, *vals;

@@ -389,6 +389,11 @@ size_t sort_scratch_bytes(uint32_t n, int key_bits)
     return 4 * ((size_t)passes * 256 + (size_t)passes * num_tiles(n) * 256 + passes);
 }
 
+cudaError_t clear_sort_scratch(void *scratch, uint32_t n, int key_bits, cudaStream_t st)
+{
+    return cudaMemsetAsync(scratch, 0, sort_scratch_bytes(n, key_bits), st);
+}
+
 cudaError_t radix_sort_pairs(uint32_t *keys, uint32_t *vals, uint32_t *keys_tmp, uint32_t *vals_tmp, uint32_t n,
                              int key_bits, const uint32_t *hist, void *scratch, uint32_t *status, cudaStream_t st,
                              SortResult *result)
@@ -402,8 +407,8 @@ cudaError_t radix_sort_pairs(uint32_t *keys, uint32_t *vals, uint32_t *keys_tmp,
     uint32_t *s_hist = static_cast<uint32_t *>(scratch);
     uint32_t *s_look = s_hist + passes * 256;
     uint32_t *s_count = s_look + (size_t)passes * tiles * 256;
-    cudaError_t e = cudaMemsetAsync(scratch, 0, sort_scratch_bytes(n, key_bits), st);
-    if (e != cudaSuccess)
+    cudaError_t e = cudaSuccess;
+    if (hist != scratch && (e = clear_sort_scratch(scratch, n, key_bits, st)) != cudaSuccess)
         return e;
     if (!hist)
     {
