@@ -2499,6 +2499,27 @@ SNCH_DEV bool ray_triangle(f3 o, f3 dir, f3 v0, f3 v1, f3 v2, float &t, float &u
 #define SNCH_RAY_POOLS 1
 #endif
 constexpr bool kRayPools = SNCH_RAY_POOLS != 0;
+// A ray's stack. An entry's distance is only compared with the hit there is, so the
+// any-hit search, which ends at its first, keeps none.
+template <bool kAny>
+struct RayStack
+{
+    uint2 e[kStackDepth];  // (node, entry distance), one access each way
+    SNCH_DEV void put(int i, uint32_t node, float d) { e[i] = make_uint2(node, __float_as_uint(d)); }
+    SNCH_DEV void get(int i, uint32_t &node, float &d) const
+    {
+        const uint2 v = e[i];
+        node = v.x;
+        d = __uint_as_float(v.y);
+    }
+};
+template <>
+struct RayStack<true>
+{
+    uint32_t e[kStackDepth];
+    SNCH_DEV void put(int i, uint32_t node, float) { e[i] = node; }
+    SNCH_DEV void get(int i, uint32_t &node, float &) const { node = e[i]; }
+};
 // one ray of the batch (batch position qi)
 template <bool kStats, bool kAny>
 SNCH_DEV void ray_query(const TreeView &t, const float *__restrict__ origins, const float *__restrict__ dirs,
@@ -2522,14 +2543,13 @@ SNCH_DEV void ray_query(const TreeView &t, const float *__restrict__ origins, co
         // The closer hit child is processed next without a trip through the
         // stack (the reference pushes it last and pops it at once, with the
         // same bound check), so the visit order is the reference's.
-        uint32_t sn[kStackDepth];
-        float sd[kStackDepth];
+        RayStack<kAny> st;
         int sp = 0;
         uint32_t node = 0;
         float nd = INFINITY;
         for (;;)
         {
-            bool next = !(nd > min_dist);
+            bool next = kAny || !(nd > min_dist);
             if (next && node >= ni)
             {
                 f3 pa, pb, pc;
@@ -2566,8 +2586,16 @@ SNCH_DEV void ray_query(const TreeView &t, const float *__restrict__ origins, co
                 if (kStats)
                     ++n_int;
                 float Ld = 0.0f, Rd = 0.0f;
-                const bool Lh = ray_box(o, inv, lb, max_dist, Ld);
-                const bool Rh = ray_box(o, inv, rb, max_dist, Rd);
+                bool Lh = ray_box(o, inv, lb, max_dist, Ld);
+                bool Rh = ray_box(o, inv, rb, max_dist, Rd);
+                if (!kAny)
+                {
+                    // beyond the hit there is: the check at its turn would skip it
+                    // (with the one-access stack: 16M rays of the 2M-triangle scene
+                    // 7.77 -> 7.61 ms)
+                    Lh = Lh && !(Ld > min_dist);
+                    Rh = Rh && !(Rd > min_dist);
+                }
                 if (Lh && Rh)
                 {
                     uint32_t closer = L, other = R;
@@ -2579,8 +2607,7 @@ SNCH_DEV void ray_query(const TreeView &t, const float *__restrict__ origins, co
                         closer = R;
                         other = L;
                     }
-                    sn[sp] = other;
-                    sd[sp] = Rd;
+                    st.put(sp, other, Rd);
                     ++sp;
                     node = closer;
                     nd = Ld;
@@ -2598,8 +2625,7 @@ SNCH_DEV void ray_query(const TreeView &t, const float *__restrict__ origins, co
             if (sp == 0)
                 break;
             --sp;
-            node = sn[sp];
-            nd = sd[sp];
+            st.get(sp, node, nd);
         }
     }
     st_out(out_hit + out_pos(t, qi, q), (uint8_t)(found ? 1 : 0));
