@@ -35,7 +35,7 @@ UNITS = [
     ("io.cu", []),
     ("scene2d.cu", ["-fmad=false"]),
 ]
-HEADERS = ["common.cuh", "coop.cuh", "internal.h", "tcgen05.cuh"]
+HEADERS = ["common.cuh", "coop.cuh", "internal.h", "tcgen05.cuh", "warp_stack.cuh"]
 
 
 def nvcc() -> str:

@@ -17,26 +17,8 @@
 // same, the answer is the minimum over the leaves reached, and exact ties are
 // resolved by leaf rank (edge key), so the order of the visits is free.
 #pragma once
+#include "warp_stack.cuh"
 
-// stack entries of a warp. A step that takes k entries adds at most k (2k
-// children), so a warp takes fewer than 32 when fewer than 32 places are left
-// below kCoopWide; one at a time adds one entry a level, and a tree over 64-bit
-// keys is at most 65 levels deep.
-constexpr int kCoopStack = 512, kCoopWide = kCoopStack - 72;
-constexpr int kCoopWarps = 2;  // per block: a block's slot is freed by its slower warp
-// Until a first candidate bounds the search, wide steps would mostly read nodes
-// that the bound then rules out, so the first steps (one per bit of the triangle
-// count, about a descent) take kCoopNarrow entries. 64,000 queries of the
-// 2M-triangle scene, nearest / silhouette: 0.44 / 0.93 ms, against 0.52 / 1.14 ms
-// with wide steps from the start; 2 or 4 entries: the same there, but small closed
-// meshes lose (1,280 triangles, silhouette, 0.57 -> 0.62 / 0.68 ms).
-constexpr int kCoopNarrow = 8;
-
-struct CoopStack
-{
-    uint32_t node[kCoopStack];
-    float md[kCoopStack];
-};
 // The edges of a step's leaves as (EdgeRec slot, tie key) items, so that lane i
 // tests the i-th edge of the warp instead of each lane looping over its own: a
 // step of 32 nodes has about 13 edges to test, in one round of loads instead of
@@ -46,44 +28,6 @@ struct CoopEdges
 {
     uint32_t slot[kCoopEdges], key[kCoopEdges];
 };
-
-// entries the next step takes from a stack of sp entries
-SNCH_DEV int coop_take(const TreeView &t, int sp, bool bounded, int step)
-{
-    const int width = bounded || step >= 32 - __clz(t.num_tris) ? 32 : kCoopNarrow;
-    return min(min(sp, width), max(1, kCoopWide - sp));
-}
-
-// pushes the children that pass (far ones first, then the near ones, lane 0's
-// near child on top); false: the stack is full
-SNCH_DEV bool coop_push(CoopStack &s, int &sp, bool pL, bool pR, uint32_t L, uint32_t R, float Lmd, float Rmd)
-{
-    const unsigned full = 0xffffffffu;
-    const bool two = pL && pR, any = pL || pR;
-    const bool l_near = two ? Lmd <= Rmd : pL;
-    const uint32_t mf = __ballot_sync(full, two), mn = __ballot_sync(full, any);
-    const int nf = __popc(mf), nn = __popc(mn);
-    if (sp + nf + nn > kCoopStack)
-        return false;
-    uint32_t above;
-    asm("mov.u32 %0, %%lanemask_gt;" : "=r"(above));
-    __syncwarp();  // every lane has read its entry
-    if (two)
-    {
-        const int at = sp + __popc(mf & above);
-        s.node[at] = l_near ? R : L;
-        s.md[at] = l_near ? Rmd : Lmd;
-    }
-    if (any)
-    {
-        const int at = sp + nf + __popc(mn & above);
-        s.node[at] = l_near ? L : R;
-        s.md[at] = l_near ? Lmd : Rmd;
-    }
-    sp += nf + nn;
-    __syncwarp();
-    return true;
-}
 
 // one query, all 32 lanes with the same arguments; (best, best_rank, nearest) is
 // the candidate the search starts with and then its answer. false: stack overflow
@@ -113,7 +57,7 @@ SNCH_DEV bool nearest_coop(const TreeView &t, f3 p, uint32_t root, float &best, 
     __syncwarp();
     for (int step = 0; sp > 0; ++step)
     {
-        const int k = coop_take(t, sp, best < INFINITY, step);
+        const int k = coop_take(t.num_tris, sp, best < INFINITY, step);
         uint32_t node = 0;
         bool act = false;
         if (lane < k)
@@ -195,20 +139,6 @@ __global__ void __launch_bounds__(32 * kCoopWarps, 16)
     nearest_coop_query(t, pts, out_idx, out_dist, seed, q, r0, r0 * r0, 0u, kInvalid, s_stack[w]);
 }
 
-// the list's next entry for this warp (words[0] entries, words[1] the next one), or
-// false at its end; an unused place comes back as query kInvalid
-SNCH_DEV bool take_deferred(const DeferArgs &d, uint4 &e)
-{
-    uint32_t i = 0;
-    if ((threadIdx.x & 31) == 0)
-        i = atomicAdd(d.count + 1, 1u);
-    i = __shfl_sync(0xffffffffu, i, 0);
-    if (i >= min(__ldcg(d.count), d.capacity))
-        return false;
-    e = __ldcg(d.list + i);
-    return true;
-}
-
 // the queries that the packets of a batch left (DeferArgs), one per warp, each from
 // the candidate it had
 __global__ void __launch_bounds__(32 * kCoopWarps, 16)
@@ -252,7 +182,7 @@ SNCH_DEV bool silhouette_coop(const TreeView &t, f3 p, bool flip, uint32_t root,
     __syncwarp();
     for (int step = 0; sp > 0; ++step)
     {
-        const int k = coop_take(t, sp, best < INFINITY, step);
+        const int k = coop_take(t.num_tris, sp, best < INFINITY, step);
         const float b2 = best * best;
         uint32_t node = 0;
         bool act = false;

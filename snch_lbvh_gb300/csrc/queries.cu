@@ -13,6 +13,7 @@
 // need more than 64 stack entries (undefined in the reference) stops, writes
 // NaN / 0xFFFFFFFF and sets kStatusStackOverflow.
 #include "internal.h"
+#include "warp_stack.cuh"
 
 namespace snch
 {
@@ -596,28 +597,6 @@ SNCH_DEV void prefetch_l1(const void *p) { asm volatile("prefetch.global.L1 [%0]
 // for silhouettes (40.9 vs 35.6 ms per 16M queries) and 11 % for nearest, so
 // they do not prefetch either.
 
-// Queries that a launch leaves to the next one, which finishes them one per warp
-// (coop.cuh) from the candidate each has: the long packets at the end of a batch
-// (leave_packet) and the long searches of a mid-sized batch (kDefer below).
-struct DeferArgs
-{
-    uint4 *list = nullptr;      // (query, candidate's distance bits, rank or key, triangle or edge); nullptr: off
-    uint32_t *count = nullptr;  // entries reserved; may pass capacity, by entries that are not in the list
-    uint32_t capacity = 0;
-};
-// lists the entry of every lane with `add` set; called by any subset of a warp
-SNCH_DEV void defer_query(const DeferArgs &d, bool add, uint4 entry)
-{
-    const uint32_t active = __activemask(), mask = __ballot_sync(active, add);
-    if (!add)
-        return;
-    const int lane = threadIdx.x & 31, leader = __ffs(mask) - 1;
-    uint32_t base = 0;
-    if (lane == leader)
-        base = atomicAdd(d.count, (uint32_t)__popc(mask));
-    base = __shfl_sync(mask, base, leader);
-    d.list[base + __popc(mask & ((1u << lane) - 1u))] = entry;
-}
 constexpr uint32_t kLaneTurns = 32;  // expansions before a query is left to the next launch
 
 // (128, 10): at most 48 registers, ten blocks per SM (silhouette: (128, 9), 56

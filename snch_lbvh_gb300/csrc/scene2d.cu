@@ -13,6 +13,7 @@
 #include <string>
 
 #include "internal.h"
+#include "warp_stack.cuh"
 
 namespace snch
 {
@@ -719,10 +720,14 @@ SNCH_DEV bool cone_test2(const C2 &bc, float2 o, const B2 &b, float dist_to_box)
 // query_device(nearest_silhouette) query.cuh:326-423 over segments, near-first (as
 // nearest2_kernel: the cone tests alone decide which leaves can be reached); also the
 // silhouette vertex (mesh vertex id) of the answer. 180,000 segments, 200k queries
-// 46.8 -> 0.49 ms.
+// 46.8 -> 0.49 ms. kDefer: a query that is not done after kLaneTurns2 expansions is left
+// to the next launch.
+constexpr uint32_t kLaneTurns2 = 64;  // 48: 160,000 queries 389 -> 460 us; 96 the same
+template <bool kDefer>
 __global__ void __launch_bounds__(128) silhouette2_kernel(Tree2 t, const float *__restrict__ pts,
                                                           const uint8_t *__restrict__ flips, int64_t n,
-                                                          float *__restrict__ out_dist, int32_t *__restrict__ out_vid)
+                                                          float *__restrict__ out_dist, int32_t *__restrict__ out_vid,
+                                                          DeferArgs defer)
 {
     const int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (q >= n)
@@ -732,6 +737,7 @@ __global__ void __launch_bounds__(128) silhouette2_kernel(Tree2 t, const float *
     float best = INFINITY;
     uint32_t best_key = 0;
     int32_t best_vert = -1;
+    bool deferred = false;
     const uint32_t ni = t.n - 1;
     if (t.n == 1)
     {
@@ -747,8 +753,14 @@ __global__ void __launch_bounds__(128) silhouette2_kernel(Tree2 t, const float *
         int sp = 0;
         uint32_t node = 0;
         bool live = true;
+        uint32_t turns = kLaneTurns2;
         while (live)
         {
+            if (kDefer && turns-- == 0)
+            {
+                deferred = true;
+                break;
+            }
             const Inner2 *rec = t.inner + node;
             const Cones2 *cr = t.inner_cones + node;
             const B2 lb = unpack_b2(__ldg(&rec->lb)), rb = unpack_b2(__ldg(&rec->rb));
@@ -804,9 +816,216 @@ __global__ void __launch_bounds__(128) silhouette2_kernel(Tree2 t, const float *
             }
         }
     }
+    if (kDefer)
+    {
+        defer_query(defer, deferred, make_uint4((uint32_t)q, __float_as_uint(best), best_key, (uint32_t)best_vert));
+        if (deferred)
+            return;
+    }
     out_dist[q] = best;
     if (out_vid)
         out_vid[q] = best_vert;
+}
+
+// The same searches, one query per warp: 32 nodes of its frontier a step (coop.cuh tells
+// why; the tests are those above, the best candidate is reduced over the warp). One lane
+// ends with its longest search: 20,000 silhouette queries of 180,000 segments take as long
+// as 100,000.
+SNCH_DEV bool nearest2_coop(const Tree2 &t, float2 p, float &best, uint32_t &best_rank, uint32_t &best_pos, CoopStack &s)
+{
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const uint32_t ni = t.n - 1;
+    __syncwarp();  // the previous query's last reads
+    if (lane == 0)
+    {
+        s.node[0] = 0;
+        s.md[0] = 0.0f;
+    }
+    int sp = 1;
+    __syncwarp();
+    for (int step = 0; sp > 0; ++step)
+    {
+        const int k = coop_take(t.n, sp, best < INFINITY, step);
+        uint32_t node = 0;
+        bool act = false;
+        if (lane < k)
+        {
+            node = s.node[sp - 1 - lane];
+            act = !(s.md[sp - 1 - lane] > best);
+        }
+        sp -= k;
+        if (__ballot_sync(full, act) == 0u)
+            continue;
+        uint32_t L = kInvalid, R = kInvalid;
+        float Lmd = INFINITY, Rmd = INFINITY, cb = best;
+        bool aL = false, aR = false;
+        uint32_t cr = best_rank, cp = best_pos;
+        if (act)
+        {
+            const Inner2 *rec = t.inner + node;
+            const B2 lb = unpack_b2(__ldg(&rec->lb)), rb = unpack_b2(__ldg(&rec->rb));
+            const uint4 ch = __ldg(&rec->ch);
+            L = ch.x;
+            R = ch.y;
+            Lmd = mindist2(lb, p);
+            Rmd = mindist2(rb, p);
+            aL = Lmd <= minmaxdist2(rb, p);
+            aR = Rmd <= minmaxdist2(lb, p);
+            if (aL && L >= ni && Lmd <= cb)
+                leaf_nearest2(t, L - ni, ch.z & kLeafRankMask, p, cb, cr, cp);
+            if (aR && R >= ni && Rmd <= cb)
+                leaf_nearest2(t, R - ni, ch.w & kLeafRankMask, p, cb, cr, cp);
+        }
+        const bool found = cp != best_pos;
+        if (__ballot_sync(full, found))
+        {
+            const uint32_t d = __reduce_min_sync(full, found ? __float_as_uint(cb) : 0xffffffffu);
+            const bool tie = found && __float_as_uint(cb) == d;
+            const uint32_t r = __reduce_max_sync(full, tie ? cr : 0u);
+            const int src = __ffs(__ballot_sync(full, tie && cr == r)) - 1;
+            best = __uint_as_float(d);
+            best_rank = r;
+            best_pos = __shfl_sync(full, cp, src);
+        }
+        if (!coop_push(s, sp, aL && L < ni && Lmd <= best, aR && R < ni && Rmd <= best, L, R, Lmd, Rmd))
+            return false;
+    }
+    return true;
+}
+__global__ void __launch_bounds__(32 * kCoopWarps, 16)
+    nearest2_coop_kernel(Tree2 t, const float *__restrict__ pts, int64_t n, uint32_t *__restrict__ out_idx,
+                         float *__restrict__ out_dist)
+{
+    __shared__ CoopStack s_stack[kCoopWarps];
+    const int w = threadIdx.x >> 5;
+    const int64_t q = blockIdx.x * (int64_t)kCoopWarps + w;
+    if (q >= n)
+        return;
+    float best = INFINITY;
+    uint32_t best_rank = 0, best_pos = kInvalid;
+    if (!nearest2_coop(t, load_pt2(pts, q), best, best_rank, best_pos, s_stack[w]))
+    {
+        if ((threadIdx.x & 31) == 0)
+            atomicOr(t.status, kStatusStackOverflow);
+        best_pos = kInvalid;
+        best = NAN;
+    }
+    if ((threadIdx.x & 31) != 0)
+        return;
+    out_idx[q] = best_pos == kInvalid ? kInvalid : __ldg(t.order + best_pos);
+    out_dist[q] = sqrtf(best);
+}
+
+SNCH_DEV bool silhouette2_coop(const Tree2 &t, float2 p, bool flip, float &best, uint32_t &best_key, int32_t &best_vert,
+                               CoopStack &s)
+{
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const uint32_t ni = t.n - 1;
+    __syncwarp();
+    if (lane == 0)
+    {
+        s.node[0] = 0;
+        s.md[0] = 0.0f;
+    }
+    int sp = 1;
+    __syncwarp();
+    for (int step = 0; sp > 0; ++step)
+    {
+        const int k = coop_take(t.n, sp, best < INFINITY, step);
+        const float b2 = best * best;
+        uint32_t node = 0;
+        bool act = false;
+        if (lane < k)
+        {
+            node = s.node[sp - 1 - lane];
+            act = !(s.md[sp - 1 - lane] > b2);
+        }
+        sp -= k;
+        if (__ballot_sync(full, act) == 0u)
+            continue;
+        uint32_t L = kInvalid, R = kInvalid, ck = best_key;
+        float Lmd = INFINITY, Rmd = INFINITY, cb = best;
+        bool hitL = false, hitR = false;
+        int32_t cv = best_vert;
+        if (act)
+        {
+            const Inner2 *rec = t.inner + node;
+            const Cones2 *cr = t.inner_cones + node;
+            const B2 lb = unpack_b2(__ldg(&rec->lb)), rb = unpack_b2(__ldg(&rec->rb));
+            const uint4 ch = __ldg(&rec->ch);
+            const C2 lc = unpack_c2(__ldg(&cr->l)), rc = unpack_c2(__ldg(&cr->r));
+            L = ch.x;
+            R = ch.y;
+            Lmd = mindist2(lb, p);
+            Rmd = mindist2(rb, p);
+            hitL = Lmd <= b2 && lc.half_angle >= 0.0f && cone_test2(lc, p, lb, Lmd);
+            hitR = Rmd <= b2 && rc.half_angle >= 0.0f && cone_test2(rc, p, rb, Rmd);
+            const uint32_t nL = hitL && L >= ni ? ch.z >> 30 : 0u, nR = hitR && R >= ni ? ch.w >> 30 : 0u;
+            for (uint32_t i = 0; i < nL + nR; ++i)
+            {
+                const bool right = i >= nL;
+                const uint32_t slot = right ? i - nL : i;
+                vertex_candidate2(t, 2 * (uint64_t)(right ? R - ni : L - ni) + slot,
+                                  ((right ? ch.w : ch.z) & kLeafRankMask) * 4u + slot, p, flip, cb, ck, cv);
+            }
+        }
+        const bool found = cv != best_vert || ck != best_key;
+        if (__ballot_sync(full, found))
+        {
+            const uint32_t d = __reduce_min_sync(full, found ? __float_as_uint(cb) : 0xffffffffu);
+            const bool tie = found && __float_as_uint(cb) == d;
+            const uint32_t order = __uint_as_float(d) > 0.0f ? ck : ~ck;
+            const uint32_t o = __reduce_max_sync(full, tie ? order : 0u);
+            const int src = __ffs(__ballot_sync(full, tie && order == o)) - 1;
+            best = __uint_as_float(d);
+            best_key = __shfl_sync(full, ck, src);
+            best_vert = __shfl_sync(full, cv, src);
+        }
+        const float b2n = best * best;
+        if (!coop_push(s, sp, hitL && L < ni && Lmd <= b2n, hitR && R < ni && Rmd <= b2n, L, R, Lmd, Rmd))
+            return false;
+    }
+    return true;
+}
+SNCH_DEV void silhouette2_coop_query(const Tree2 &t, const float *__restrict__ pts, const uint8_t *__restrict__ flips,
+                                     float *__restrict__ out_dist, int32_t *__restrict__ out_vid, int64_t q, float best,
+                                     uint32_t best_key, int32_t best_vert, CoopStack &s)
+{
+    const bool flip = flips ? __ldg(flips + q) != 0 : false;
+    if (!silhouette2_coop(t, load_pt2(pts, q), flip, best, best_key, best_vert, s))
+    {
+        if ((threadIdx.x & 31) == 0)
+            atomicOr(t.status, kStatusStackOverflow);
+        best = NAN;
+        best_vert = -1;
+    }
+    if ((threadIdx.x & 31) != 0)
+        return;
+    out_dist[q] = best;
+    if (out_vid)
+        out_vid[q] = best_vert;
+}
+__global__ void __launch_bounds__(32 * kCoopWarps, 16)
+    silhouette2_coop_kernel(Tree2 t, const float *__restrict__ pts, const uint8_t *__restrict__ flips, int64_t n,
+                            float *__restrict__ out_dist, int32_t *__restrict__ out_vid)
+{
+    __shared__ CoopStack s_stack[kCoopWarps];
+    const int w = threadIdx.x >> 5;
+    const int64_t q = blockIdx.x * (int64_t)kCoopWarps + w;
+    if (q < n)
+        silhouette2_coop_query(t, pts, flips, out_dist, out_vid, q, INFINITY, 0u, -1, s_stack[w]);
+}
+__global__ void __launch_bounds__(32 * kCoopWarps, 16)
+    silhouette2_finish_kernel(Tree2 t, const float *__restrict__ pts, const uint8_t *__restrict__ flips,
+                              float *__restrict__ out_dist, int32_t *__restrict__ out_vid, DeferArgs d)
+{
+    __shared__ CoopStack s_stack[kCoopWarps];
+    uint4 e;
+    while (take_deferred(d, e))
+        silhouette2_coop_query(t, pts, flips, out_dist, out_vid, (int64_t)e.x, __uint_as_float(e.y), e.z, (int32_t)e.w,
+                               s_stack[threadIdx.x >> 5]);
 }
 
 // intersects_d(ray<float,2>) aabb.cuh:366-390
@@ -1117,6 +1336,43 @@ int check2(snch_scene2_t s, int64_t n, std::initializer_list<const void *> ptrs)
 }
 }  // namespace
 
+namespace
+{
+// Batches of up to kCoopDirect2 queries are searched a warp each, so that they do not wait
+// for the longest search of one lane; silhouette batches of up to kLanesFirst2 a lane each
+// at first, and the long ones then a warp each; larger ones keep the chip busy with a lane
+// each. Measured, a lane each / as chosen, us: nearest, 20,000 queries of 180,000 segments
+// 128 / 113, 26,000 of 1,800 143 / 89; silhouettes 394 / 166, 218 / 133, 130,000 of 180,000
+// 460 / 361 (200,000: 516 / 547; nearest with lanes first, 130,000: 179 / 195).
+constexpr int64_t kCoopDirect2 = 24576, kLanesFirst2 = 131072;
+// both(list, blocks) launches the lanes and the warps that finish their list
+template <typename Both>
+cudaError_t launch_lanes_first2(int64_t n, cudaStream_t st, Both both)
+{
+    int dev = 0, sms = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess)
+        e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    char *scratch = nullptr;
+    if (e != cudaSuccess ||
+        (e = scratch_alloc_raw(reinterpret_cast<void **>(&scratch), 256 + 16 * (size_t)n, st)) != cudaSuccess)
+        return e;
+    DeferArgs d;
+    d.count = reinterpret_cast<uint32_t *>(scratch);
+    d.list = reinterpret_cast<uint4 *>(scratch + 256);
+    d.capacity = (uint32_t)n;
+    e = cudaMemsetAsync(scratch, 0, 8, st);
+    if (e == cudaSuccess)
+    {
+        both(d, 16 * (unsigned)sms);
+        note_launch(2);
+        e = cudaGetLastError();
+    }
+    const cudaError_t f = cudaFreeAsync(scratch, st);
+    return e != cudaSuccess ? e : f;
+}
+}  // namespace
+
 extern "C" {
 
 int snch_scene2_create(const float *verts_xy, int64_t nv, const int32_t *segs, int64_t ns, snch_scene2_t *out)
@@ -1291,7 +1547,12 @@ int snch_scene2_query_nearest(snch_scene2_t s, const float *pts, int64_t n, uint
     int rc = check2(s, n, {pts, idx, dist});
     if (rc != SNCH_OK || n == 0)
         return rc;
-    nearest2_kernel<<<blocks(n, 128), 128, 0, S2(stream)>>>(s->tree(), pts, n, idx, dist);
+    const Tree2 t = s->tree();
+    cudaStream_t st = S2(stream);
+    if (t.n > 1 && n <= kCoopDirect2)
+        nearest2_coop_kernel<<<blocks(n, kCoopWarps), 32 * kCoopWarps, 0, st>>>(t, pts, n, idx, dist);
+    else
+        nearest2_kernel<<<blocks(n, 128), 128, 0, st>>>(t, pts, n, idx, dist);
     note_launch();
     SNCH2_CUDA(cudaGetLastError());
     return SNCH_OK;
@@ -1303,7 +1564,20 @@ int snch_scene2_query_silhouette(snch_scene2_t s, const float *pts, const uint8_
     int rc = check2(s, n, {pts, dist});
     if (rc != SNCH_OK || n == 0)
         return rc;
-    silhouette2_kernel<<<blocks(n, 128), 128, 0, S2(stream)>>>(s->tree(), pts, flip, n, dist, vertex);
+    const Tree2 t = s->tree();
+    cudaStream_t st = S2(stream);
+    if (t.n > 1 && n > kCoopDirect2 && n <= kLanesFirst2)
+    {
+        SNCH2_CUDA(launch_lanes_first2(n, st, [&](const DeferArgs &d, unsigned g) {
+            silhouette2_kernel<true><<<blocks(n, 128), 128, 0, st>>>(t, pts, flip, n, dist, vertex, d);
+            silhouette2_finish_kernel<<<g, 32 * kCoopWarps, 0, st>>>(t, pts, flip, dist, vertex, d);
+        }));
+        return SNCH_OK;
+    }
+    if (t.n > 1 && n <= kCoopDirect2)
+        silhouette2_coop_kernel<<<blocks(n, kCoopWarps), 32 * kCoopWarps, 0, st>>>(t, pts, flip, n, dist, vertex);
+    else
+        silhouette2_kernel<false><<<blocks(n, 128), 128, 0, st>>>(t, pts, flip, n, dist, vertex, DeferArgs());
     note_launch();
     SNCH2_CUDA(cudaGetLastError());
     return SNCH_OK;

@@ -98,3 +98,37 @@ def test_batched_scene(snch, n):
     p, f = points(n, seed=5)
     m = torch.randint(0, len(meshes), (n,), generator=torch.Generator().manual_seed(1), dtype=torch.int32).cuda()
     same(*both_forms(snch, s, lambda: s.query_nearest_batch(m, p) + s.query_silhouette_batch(m, p, f)))
+
+
+@pytest.mark.parametrize("segments", [2, 3, 40, 20_000])
+@pytest.mark.parametrize("n", [1, 24_576, 24_577, 131_072, 131_073])
+def test_2d_forms_agree(segments, n):
+    """A warp per query, lanes then warps, and a lane per query: one batch of n queries
+    against the same queries in batches of 1,000 (a warp each), bit for bit (2D boxes are
+    inflated, so the bound never cuts off an equal candidate)."""
+    import snch_lbvh_gb300 as snch
+    import torch
+    rng = np.random.default_rng(segments)
+    k = segments
+    a = np.sort(rng.random(k)) * 2 * np.pi
+    r = 5.0 * (1 + 0.05 * rng.standard_normal(k))
+    v = np.stack([r * np.cos(a), r * np.sin(a)], 1).astype(np.float32)
+    i = np.arange(k)
+    sg = np.stack([i, (i + 1) % k], 1)[: k if k > 2 else k - 1].astype(np.int32)
+    sg = np.concatenate([sg, sg[:1]]) if k == 2 else sg
+    s = snch.Scene2(v, sg)
+    s.build()
+    p = ((rng.random((n, 2)) - 0.5) * 14).astype(np.float32)
+    p[: min(n, k)] = v[: min(n, k)]  # on vertices: distance 0 and ties of two segments
+    p, flip = torch.from_numpy(p).cuda(), torch.from_numpy((rng.random(n) < 0.5).astype(np.uint8)).cuda()
+    part = slice(max(0, n - 1000), n), slice(0, min(n, 1000))
+    idx, dist = s.query_nearest(p)
+    sd, sv = s.query_silhouette(p, flip)
+    for w in part:
+        bi, bd = s.query_nearest(p[w].contiguous())
+        bsd, bsv = s.query_silhouette(p[w].contiguous(), flip[w].contiguous())
+        assert torch.equal(dist[w].view(torch.int32), bd.view(torch.int32))
+        assert torch.equal(sd[w].view(torch.int32), bsd.view(torch.int32))
+        assert torch.equal(idx[w], bi)
+        assert torch.equal(sv[w], bsv)
+    assert s.device_status() == 0
