@@ -321,6 +321,20 @@ cudaError_t snch::scratch_alloc_raw(void **pp, size_t bytes, cudaStream_t st)
 }
 
 
+char *snch::optional_scratch(size_t bytes, cudaStream_t st, bool in_capture)
+{
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    void *p = nullptr;
+    if ((!in_capture && (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone)) ||
+        scratch_alloc_raw(&p, bytes, st) != cudaSuccess)
+    {
+        cudaGetLastError();
+        return nullptr;
+    }
+    return static_cast<char *>(p);
+}
+
+
 namespace
 {
 template <typename T>

@@ -143,6 +143,10 @@ cudaError_t launch_enumerate(const TreeView &t, bool line, const float *q0, cons
 // (kept mapped between calls; cudaMallocAsync under stream capture). Free with
 // cudaFreeAsync on the same stream.
 cudaError_t scratch_alloc_raw(void **p, size_t bytes, cudaStream_t st);
+// Scratch that makes a search faster but that it can do without: nullptr if there is no
+// memory for it, or, unless in_capture, if the stream is being captured (a graph without
+// allocations can be cloned, updated and embedded).
+char *optional_scratch(size_t bytes, cudaStream_t st, bool in_capture);
 // The queries of a seeded batch whose fail_flag is set, listed in batch order
 // (order[i], or i without an order) with their count, all on the device.
 size_t failed_list_scratch_bytes(int64_t n);

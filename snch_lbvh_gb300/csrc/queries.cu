@@ -627,7 +627,7 @@ __global__ void __launch_bounds__(kBlock, 1280 / kBlock) nearest_fast_kernel(Tre
         best = r0 * r0;
     }
     bool deferred = false;
-    uint32_t budget = kDefer ? kLaneTurns : seed.cap ? seed.cap : 0xFFFFFFFFu;
+    uint32_t budget = kDefer && defer.list ? kLaneTurns : !kDefer && seed.cap ? seed.cap : 0xFFFFFFFFu;
     const uint32_t ni = t.num_tris - 1;
     const QueryRoot qr = query_root(t, q);
     if (qr.node == kInvalid)
@@ -860,7 +860,7 @@ __global__ void __launch_bounds__(kBlock, 1152 / kBlock) silhouette_fast_kernel(
     uint32_t best_key = 0;
     int32_t best_edge = -1;
     bool deferred = false;
-    uint32_t budget = kDefer ? kLaneTurns : seed.cap ? seed.cap : 0xFFFFFFFFu;
+    uint32_t budget = kDefer && defer.list ? kLaneTurns : !kDefer && seed.cap ? seed.cap : 0xFFFFFFFFu;
     const uint32_t ni = t.num_tris - 1;
     const QueryRoot qr = query_root(t, q);
     if (qr.node == kInvalid)
@@ -3426,11 +3426,12 @@ cudaError_t launch_deferring(void (*kernel)(KArgs...), int64_t n, cudaStream_t s
     DeferArgs d;
     d.capacity = (uint32_t)std::min<int64_t>((n + 31) / 32 * 32, in_flight);
     constexpr size_t head = (kWorkBytes + 8 + 255) / 256 * 256;  // counter, pools, list count, list position
-    char *scratch = nullptr;
-    if ((e = scratch_alloc_raw(reinterpret_cast<void **>(&scratch), head + 16 * (size_t)d.capacity, st)) != cudaSuccess)
+    char *scratch = optional_scratch(head + 16 * (size_t)d.capacity, st, true);
+    if (scratch)
+        d.list = reinterpret_cast<uint4 *>(scratch + head);
+    else if ((e = scratch_alloc_raw(reinterpret_cast<void **>(&scratch), head, st)) != cudaSuccess)
         return e;
     d.count = reinterpret_cast<uint32_t *>(scratch + kWorkBytes);
-    d.list = reinterpret_cast<uint4 *>(scratch + head);
     e = cudaMemsetAsync(scratch, 0, head, st);
     if (e == cudaSuccess)
     {
@@ -3438,7 +3439,7 @@ cudaError_t launch_deferring(void (*kernel)(KArgs...), int64_t n, cudaStream_t s
         note_launch();
         e = cudaGetLastError();
     }
-    if (e == cudaSuccess)
+    if (e == cudaSuccess && d.list)
     {
         finish(d, 16 * sms);
         note_launch();
@@ -3448,19 +3449,25 @@ cudaError_t launch_deferring(void (*kernel)(KArgs...), int64_t n, cudaStream_t s
     return e != cudaSuccess ? e : f;
 }
 // One query per lane, whose long ones end in a second launch: launch(d) and finish(d,
-// blocks) enqueue the two
+// blocks) enqueue the two; without memory for the list the first one alone, all of it
 template <typename Launch, typename Finish>
-cudaError_t launch_lanes_deferring(int64_t n, cudaStream_t st, Launch launch, Finish finish)
+cudaError_t launch_lanes_deferring(int64_t n, cudaStream_t st, bool ordered, Launch launch, Finish finish)
 {
     int dev = 0, sms = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess)
         e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    char *scratch = nullptr;
-    if (e != cudaSuccess ||
-        (e = scratch_alloc_raw(reinterpret_cast<void **>(&scratch), 256 + 16 * (size_t)n, st)) != cudaSuccess)
+    if (e != cudaSuccess)
         return e;
     DeferArgs d;
+    // an ordered batch has scratch in the capture already
+    char *scratch = optional_scratch(256 + 16 * (size_t)n, st, ordered);
+    if (!scratch)
+    {
+        launch(d);
+        note_launch();
+        return cudaGetLastError();
+    }
     d.count = reinterpret_cast<uint32_t *>(scratch);
     d.list = reinterpret_cast<uint4 *>(scratch + 256);
     d.capacity = (uint32_t)n;
@@ -3633,7 +3640,7 @@ cudaError_t launch_nearest(const TreeView &t0, const float *pts, int64_t n, uint
     else if (coop && n > kCoopDirect)
     {
         e = launch_lanes_deferring(
-            n, st,
+            n, st, t.order != nullptr,
             [&](const DeferArgs &d) {
                 nearest_fast_kernel<false, 128, true><<<grid_for(n, 128), 128, 0, st>>>(t, pts, n, idx, dist, nullptr,
                                                                                        seed, d);
@@ -3746,7 +3753,7 @@ cudaError_t launch_silhouette(const TreeView &t0, const float *pts, const uint8_
     else if (coop && n > kCoopDirect)
     {
         e = launch_lanes_deferring(
-            n, st,
+            n, st, t.order != nullptr,
             [&](const DeferArgs &d) {
                 silhouette_fast_kernel<false, 128, true>
                     <<<grid_for(n, 128), 128, 0, st>>>(t, pts, flip, n, dist, edge, nullptr, seed, d);

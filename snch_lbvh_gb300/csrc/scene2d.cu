@@ -753,7 +753,7 @@ __global__ void __launch_bounds__(128) silhouette2_kernel(Tree2 t, const float *
         int sp = 0;
         uint32_t node = 0;
         bool live = true;
-        uint32_t turns = kLaneTurns2;
+        uint32_t turns = kDefer && defer.list ? kLaneTurns2 : 0xFFFFFFFFu;
         while (live)
         {
             if (kDefer && turns-- == 0)
@@ -1345,26 +1345,33 @@ namespace
 // 128 / 113, 26,000 of 1,800 143 / 89; silhouettes 394 / 166, 218 / 133, 130,000 of 180,000
 // 460 / 361 (200,000: 516 / 547; nearest with lanes first, 130,000: 179 / 195).
 constexpr int64_t kCoopDirect2 = 24576, kLanesFirst2 = 131072;
-// both(list, blocks) launches the lanes and the warps that finish their list
-template <typename Both>
-cudaError_t launch_lanes_first2(int64_t n, cudaStream_t st, Both both)
+// launch(d): the lanes, finish(d, blocks): the warps that finish their list; without memory
+// for the list, or under capture (no allocation in the graph, as before), the lanes alone
+template <typename Launch, typename Finish>
+cudaError_t launch_lanes_first2(int64_t n, cudaStream_t st, Launch launch, Finish finish)
 {
     int dev = 0, sms = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess)
         e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    char *scratch = nullptr;
-    if (e != cudaSuccess ||
-        (e = scratch_alloc_raw(reinterpret_cast<void **>(&scratch), 256 + 16 * (size_t)n, st)) != cudaSuccess)
+    if (e != cudaSuccess)
         return e;
     DeferArgs d;
+    char *scratch = optional_scratch(256 + 16 * (size_t)n, st, false);
+    if (!scratch)
+    {
+        launch(d);
+        note_launch();
+        return cudaGetLastError();
+    }
     d.count = reinterpret_cast<uint32_t *>(scratch);
     d.list = reinterpret_cast<uint4 *>(scratch + 256);
     d.capacity = (uint32_t)n;
     e = cudaMemsetAsync(scratch, 0, 8, st);
     if (e == cudaSuccess)
     {
-        both(d, 16 * (unsigned)sms);
+        launch(d);
+        finish(d, 16 * (unsigned)sms);
         note_launch(2);
         e = cudaGetLastError();
     }
@@ -1568,10 +1575,14 @@ int snch_scene2_query_silhouette(snch_scene2_t s, const float *pts, const uint8_
     cudaStream_t st = S2(stream);
     if (t.n > 1 && n > kCoopDirect2 && n <= kLanesFirst2)
     {
-        SNCH2_CUDA(launch_lanes_first2(n, st, [&](const DeferArgs &d, unsigned g) {
-            silhouette2_kernel<true><<<blocks(n, 128), 128, 0, st>>>(t, pts, flip, n, dist, vertex, d);
-            silhouette2_finish_kernel<<<g, 32 * kCoopWarps, 0, st>>>(t, pts, flip, dist, vertex, d);
-        }));
+        SNCH2_CUDA(launch_lanes_first2(
+            n, st,
+            [&](const DeferArgs &d) {
+                silhouette2_kernel<true><<<blocks(n, 128), 128, 0, st>>>(t, pts, flip, n, dist, vertex, d);
+            },
+            [&](const DeferArgs &d, unsigned g) {
+                silhouette2_finish_kernel<<<g, 32 * kCoopWarps, 0, st>>>(t, pts, flip, dist, vertex, d);
+            }));
         return SNCH_OK;
     }
     if (t.n > 1 && n <= kCoopDirect2)

@@ -132,3 +132,40 @@ def test_2d_forms_agree(segments, n):
         assert torch.equal(idx[w], bi)
         assert torch.equal(sv[w], bsv)
     assert s.device_status() == 0
+
+
+@pytest.mark.parametrize("n", [30_000, 100_000])
+def test_forms_under_capture(snch, n):
+    """A captured batch of a size that would be finished by a second launch: the replayed
+    answers are the direct ones, bit for bit, and ids up to exact ties at distance equal."""
+    import torch
+    v, f = mesh(3)
+    s = snch.Scene(v, f)
+    s.compute_silhouettes()
+    s.build_bvh()
+    p, flip = points(n, seed=8)
+    a = np.linspace(0, 2 * np.pi, 500, endpoint=False)
+    s2 = snch.Scene2(np.stack([np.cos(a), np.sin(a)], 1).astype(np.float32) * (1 + 0.01 * np.sin(40 * a))[:, None].astype(np.float32),
+                     np.stack([np.arange(500), (np.arange(500) + 1) % 500], 1).astype(np.int32))
+    s2.build()
+    p2 = p[:, :2].contiguous()
+
+    def everything():
+        st = torch.cuda.current_stream()
+        return (s.query_nearest(p, stream=st) + s.query_silhouette(p, flip, stream=st) +
+                s2.query_nearest(p2, stream=st) + s2.query_silhouette(p2, flip, stream=st))
+
+    direct = [x.clone() for x in everything()]
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        out = everything()
+    for x in out:
+        x.zero_()
+    g.replay()
+    torch.cuda.synchronize()
+    for k in (1, 2, 5, 6):  # distances
+        assert torch.equal(out[k].view(torch.int32), direct[k].view(torch.int32)), k
+    for k in (0, 3, 4, 7):
+        assert (out[k] == direct[k]).float().mean().item() > 0.999, k
+    assert s.device_status() == 0 and s2.device_status() == 0
