@@ -42,8 +42,8 @@ sys.path.insert(0, ROOT)
 METRIC = ("queries/sec (walk-on-stars query set: nearest, silhouette, ray, sphere sample) on the 2M-triangle "
           "scene")
 FULL = {"near": 16_000_000, "sil": 16_000_000, "ray": 16_000_000, "smp": 4_000_000}
-# kernels the default configuration runs for each query type (Morton-ordered
-# 16M-query batches, 8 queries per triangle: nearest and silhouette batches
+# kernels the default configuration runs for each query type (ordered 16M-query
+# batches, 8 queries per triangle: nearest and silhouette batches
 # run as persistent warp packets, rays as warps taking 32 rays at a time)
 KERNEL_OF = {"near": "nearest_packet_persistent_kernel", "sil": "silhouette_packet_persistent_kernel",
              "ray": "ray_pool_kernel", "smp": "sample_kernel"}

@@ -109,7 +109,9 @@ int snch_get_bvh_view(snch_scene_t scene, snch_bvh_view *out_view);
  *   inner[N-1], 64 B: (Lup.xyz, Llo.x) (Llo.yz, Rup.xy) (Rup.z, Rlo.xyz)
  *                     (bits L, bits R, bits Linfo, bits Rinfo); children are
  *                     node ids (internal < N-1 <= leaf N-1+j for sorted leaf j);
- *                     a leaf child's info = depth-first rank | owned edges << 30
+ *                     a leaf child's info = depth-first rank | owned edges << 30; an
+ *                     internal child's: 1 = its cone test always passes, 2 = it never
+ *                     does, 0 = read its cone
  *   inner_cones[N-1], 48 B: (L.axis, L.half) (L.radius, R.axis) (R.half, R.radius, 0, 0)
  *   leaves[N], 48 B:  (a.xyz, bits original index) (b.xyz, bits owned edges) (c.xyz, bits rank)
  *   edges[3N], 64 B:  owned silhouette edge k of sorted leaf j at 3j+k:
@@ -205,9 +207,10 @@ int snch_set_traversal(snch_scene_t scene, int mode);
  * result, and every option below changes only how fast an answer comes):
  *   SNCH_OPT_TRAVERSAL        SNCH_TRAVERSAL_NEAR_FIRST (default) / _REFERENCE_ORDER
  *   SNCH_OPT_QUERY_ORDER      1 (default): nearest, silhouette and ray batches are
- *                             answered in the Morton order of their query points
- *                             (results still land at their input positions and do not
- *                             change); 0: input order. Sphere draws always run in input
+ *                             answered in the order of their query points along a
+ *                             space-filling curve (Hilbert; rays Morton); results
+ *                             still land at their input positions and do not
+ *                             change; 0: input order. Sphere draws always run in input
  *                             order: their single descent gains less from the order
  *                             than the sort costs (4M draws: 0.77 ms against 0.93).
  *   SNCH_OPT_ORDER_MIN_BATCH  smallest batch that is reordered (default 65536) */
@@ -317,7 +320,7 @@ int snch_set_traversal(snch_scene_t scene, int mode);
  *                             slower on 16M rays with tmax log-uniform over three decades:
  *                             the lost spatial coherence costs more). Same results. */
 #define SNCH_OPT_RAY_ORDER 22
-/*   SNCH_OPT_ORDER_BITS       bits of a query's Morton code (plain scenes) that order a
+/*   SNCH_OPT_ORDER_BITS       bits of a query's curve code (plain scenes) that order a
  *                             batch: 12 to 30, default 24 (a 256^3 grid, sorted in three
  *                             radix passes; measured on 16M-query batches of the
  *                             2M-triangle scene: 0.4 % faster per step than 30 bits in four
