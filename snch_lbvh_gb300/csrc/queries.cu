@@ -2964,6 +2964,7 @@ __global__ void __launch_bounds__(128) sample_kernel(TreeView t, const float *__
             // and a division each) and the two divisions of the choice are not computed.
             // A weight is 0, which ends the draw, only if the squared distance overflows;
             // u outside [0, 1), after rounding or by the caller, takes the general form.
+            // 4M draws and their points 0.776 -> 0.758 ms.
             const bool Lh = sphere_box(c, rad, lb), Rh = sphere_box(c, rad, rb);
             if (!(Lh || Rh))
                 break;
