@@ -632,6 +632,12 @@ SNCH_DEV Cone ldcg_cone(const Cone *p)
 // reads a level, and the gathers of the leaves wait for few warps. Here 250 + 204 + 66
 // us (one kernel for all three: 770 us, held up by the walks at its end).
 constexpr int kRefitLeaves = 256;
+// A tree of up to so many leaves is one block's: nothing is left for refit_top_kernel, and
+// it is not launched (tree build of 256 triangles 52 -> 49 us). A block of 1,024 costs such
+// a tree less than the exits of two to four blocks of 256 do (306 triangles 71 -> 49 us, 992
+// 79 -> 60); larger trees lose with such blocks (11,990 triangles 120 -> 127 us, 399,424
+// 273 -> 288).
+constexpr int kRefitWide = 1024;
 
 // scratch in the space of the centroids, which are dead after the Morton codes
 struct RefitScratch
@@ -648,9 +654,9 @@ SNCH_DEV RefitScratch refit_scratch(const BuildArgs &a)
 
 // the internal node at index j, with w = 1 if its leaves, and so the slots of its
 // children, all lie in the block of first leaf b0; size: leaves under it
+template <uint32_t B>
 SNCH_DEV uint4 block_node(const BuildArgs &a, uint32_t j, uint32_t b0, uint32_t &size)
 {
-    constexpr uint32_t B = kRefitLeaves;
     const uint32_t ni = a.num_tris - 1;
     size = 0;
     if (j >= ni)
@@ -710,7 +716,7 @@ __global__ void __launch_bounds__(kRefitLeaves, 4) leaf_records_kernel(BuildArgs
     const bool leaf = orig < n;  // otherwise past the end, or after a failed sort (status bit set)
     const uint32_t parent = leaf && n > 1 ? a.nodes[ni + j].parent : kInvalid;
     uint32_t size;
-    const uint4 node = block_node(a, j, b0, size);
+    const uint4 node = block_node<B>(a, j, b0, size);
     s_node[t] = node;
     s_size[t] = size;
     __syncthreads();
@@ -757,13 +763,25 @@ __global__ void __launch_bounds__(kRefitLeaves, 4) leaf_records_kernel(BuildArgs
 // consecutive threads (the merge's acosf, sinf and cosf run in full warps; a walk per
 // leaf loses half of its lanes at every level). Bound by the chain of about 15 such merges;
 // 6 blocks per SM: 204 us, 5 / 4: 212 / 224.
-__global__ void __launch_bounds__(kRefitLeaves, 6) refit_kernel(BuildArgs a)
+template <uint32_t B>
+struct RefitShared
 {
-    constexpr uint32_t B = kRefitLeaves;
-    __shared__ float s_val[11][2 * B];  // box and cone: slot t = leaf t, B + t = internal node t
-    __shared__ uint4 s_node[B];
-    __shared__ uint32_t s_info[B], s_arrived[B], s_list[2][B], s_exit[B];
-    __shared__ uint32_t s_count[2], s_exits, s_exit_base;
+    uint4 node[B];
+    float val[11][2 * B];  // box and cone: slot t = leaf t, B + t = internal node t
+    uint32_t info[B], arrived[B], list[2][B], exit[B];
+    uint32_t count[2], exits, exit_base;
+};
+template <uint32_t B>
+__global__ void __launch_bounds__(B, B == kRefitLeaves ? 6 : 1) refit_kernel(BuildArgs a)
+{
+    extern __shared__ uint4 s_raw[];
+    RefitShared<B> &sh = *reinterpret_cast<RefitShared<B> *>(s_raw);
+    auto &s_val = sh.val;
+    auto &s_node = sh.node;
+    auto &s_info = sh.info, &s_arrived = sh.arrived, &s_exit = sh.exit;
+    auto &s_list = sh.list;
+    auto &s_count = sh.count;
+    uint32_t &s_exits = sh.exits, &s_exit_base = sh.exit_base;
     const uint32_t n = a.num_tris, ni = n - 1;
     const uint32_t b0 = blockIdx.x * B, t = threadIdx.x, j = b0 + t;
     const RefitScratch scratch = refit_scratch(a);
@@ -804,7 +822,7 @@ __global__ void __launch_bounds__(kRefitLeaves, 6) refit_kernel(BuildArgs a)
     };
 
     uint32_t size;
-    s_node[t] = block_node(a, j, b0, size);
+    s_node[t] = block_node<B>(a, j, b0, size);
     s_arrived[t] = 0;
     if (t < 2)
         s_count[t] = 0;
@@ -1212,9 +1230,23 @@ cudaError_t launch_build_back(const BuildArgs &a, cudaStream_t st)
     note_launch();
     if (n > 1)
     {
-        refit_kernel<<<blocks, kRefitLeaves, 0, st>>>(a);
-        refit_top_kernel<<<(16 * blocks + 127) / 128, 128, 0, st>>>(a);  // about 16 exits a block
-        note_launch(2);
+        if (n <= kRefitLeaves)
+            refit_kernel<kRefitLeaves><<<1, kRefitLeaves, sizeof(RefitShared<kRefitLeaves>), st>>>(a);
+        else if (n <= kRefitWide)
+        {
+            const cudaError_t e = cudaFuncSetAttribute(refit_kernel<kRefitWide>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                       (int)sizeof(RefitShared<kRefitWide>));
+            if (e != cudaSuccess)
+                return e;
+            refit_kernel<kRefitWide><<<1, kRefitWide, sizeof(RefitShared<kRefitWide>), st>>>(a);
+        }
+        else
+        {
+            refit_kernel<kRefitLeaves><<<blocks, kRefitLeaves, sizeof(RefitShared<kRefitLeaves>), st>>>(a);
+            refit_top_kernel<<<(16 * blocks + 127) / 128, 128, 0, st>>>(a);  // about 16 exits a block
+            note_launch();
+        }
+        note_launch();
     }
     return cudaGetLastError();
 }

@@ -143,3 +143,10 @@ def test_view_objects(snch, oracle_mod, n):
     e = device_words(int(ptrs[0, 1]), len(orc.edge_verts), 8)
     np.testing.assert_array_equal(e[:, :4], orc.edge_verts)
     assert (e[:, 4:6].copy().view(np.uint64) == verts.value).all()
+
+
+@pytest.mark.parametrize("make", [grid, soup])
+@pytest.mark.parametrize("n", [769, 1023, 1024, 1025])
+def test_one_block_trees(snch, oracle_mod, make, n):
+    """Trees that one block of the refit covers, and the first that it does not."""
+    test_topology_and_tree(snch, oracle_mod, make, n)
