@@ -3359,6 +3359,10 @@ inline bool coop_ok(const TreeView &t, int packet, int width, int block, bool pe
 // 31.7 / 31.1 / 37.0 ms, 32 28.7.
 constexpr int64_t kCoopDirect = 24576;
 constexpr int64_t kCoopNearestMax = 98304, kCoopSilhouetteMax = 131072;
+// Sparse silhouette batches, at most a query per 8 triangles, keep to it longer: their
+// packets of 32 neighbours reach far (2M-triangle scene, packets / lanes first, ms:
+// 140,000 queries 1.91 / 1.42, 220,000 2.62 / 2.13, 300,000 3.00 / 2.78, 400,000 3.47 / 3.55).
+constexpr int64_t kCoopSilhouetteSparseMax = 1 << 18;
 // the wide searches serve near-first, one-thread-per-query, uncapped launches
 // over a tree whose wide records of that width exist
 inline bool wide_ok(const TreeView &t, int width, bool persistent, const SeedArgs &seed)
@@ -3683,7 +3687,8 @@ cudaError_t launch_silhouette(const TreeView &t0, const float *pts, const uint8_
         return cudaSuccess;
     TreeView t = t0;
     const bool persistent = (t.persistent & 2) != 0;
-    const bool coop = !stats && n <= kCoopSilhouetteMax &&
+    const bool coop = !stats &&
+                      n <= (8 * (uint64_t)n <= t.num_tris ? kCoopSilhouetteSparseMax : kCoopSilhouetteMax) &&
                       coop_ok(t, t.packet_sil, t.width_sil, t.block_sil, persistent, seed);
     const bool packets = !coop && packet_ok(t, t.packet_sil, t.width_sil, seed);
     const bool wide = !packets && wide_ok(t, t.width_sil, persistent, seed);

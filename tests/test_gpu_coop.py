@@ -169,3 +169,23 @@ def test_forms_under_capture(snch, n):
     for k in (0, 3, 4, 7):
         assert (out[k] == direct[k]).float().mean().item() > 0.999, k
     assert s.device_status() == 0 and s2.device_status() == 0
+
+
+@pytest.mark.parametrize("n", [131_073, 149_440, 149_441])
+def test_sparse_silhouette_batches(snch, n):
+    """Around the sizes at which a batch is sparse enough for lanes and then warps: the
+    one-query-per-lane answers, bit for bit, ids up to exact ties."""
+    import torch
+    from snch_lbvh_gb300 import meshes
+    v, f = meshes.torus(0.8, 0.3, 1868, 320)[:2]
+    assert len(f) == 8 * 149_440
+    s = snch.Scene(v.astype(np.float32), f)
+    s.compute_silhouettes()
+    s.build_bvh()
+    p, flip = points(n, seed=3)
+    a = s.query_silhouette(p, flip)
+    s.set_option(snch.OPT_PACKET, 0)
+    b = s.query_silhouette(p, flip)
+    assert torch.equal(a[0].view(torch.int32), b[0].view(torch.int32))
+    assert (a[1] == b[1]).float().mean().item() > 0.999
+    assert s.device_status() == 0
