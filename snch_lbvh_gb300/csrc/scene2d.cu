@@ -8,7 +8,8 @@
 // reference's expression order, so topology, Morton codes, tree and boxes are
 // bit-identical to the reference's; acosf / asinf / atan2f / logf / sinf / cosf
 // are CUDA's. Rays and circle samples replay the reference's traversal order; the
-// nearest and silhouette searches go near-first and give its answers (see there).
+// nearest and silhouette searches go near-first where that gives its answers, and replay
+// it elsewhere (in_order2).
 #include <algorithm>
 #include <string>
 
@@ -542,15 +543,35 @@ SNCH_DEV float closest_point_segment2_sq(float2 pa, float2 pb, float2 x)
 }
 SNCH_DEV float2 load_pt2(const float *p, int64_t q) { return f2(__ldg(p + 2 * q), __ldg(p + 2 * q + 1)); }
 
-// query_device(nearest) query.cuh:239-318 over segments, near-first. The reference
-// visits its stack in a fixed order; its answer is the minimum over the leaves its
-// child tests (mindist against the sibling's minmaxdist) let it reach, the last one
-// visited among equals. Those tests depend on the node and the query alone and are
-// kept (a 2D box is inflated by 1e-3, so that the sibling test can cut off a nearer
-// segment: dropping it would change answers); pruning by the best so far never
-// removes a leaf at the minimum, so any order reaches the same minimum, and equals
-// are resolved by leaf rank. Bound by dependent reads, one record a step:
-// 180,000 segments, 200k queries 2.26 -> 0.18 ms.
+// ---- where near-first gives the reference's answers
+// The reference takes its stack in a fixed order and prunes stack entries by the best so
+// far, but evaluates every leaf child of a node that it expands. Its child tests (nearest:
+// mindist against the sibling's minmaxdist; silhouette: the cone) depend on the node and
+// the query alone; the near-first searches keep them (a 2D box is inflated by 1e-3, so that
+// the sibling test can cut off a nearer segment: dropping it would change answers). Its
+// answer is the minimum over the leaves that those tests reach, the last one visited among
+// equals, if no leaf at the minimum is ever pruned; any order then gives the same, with
+// equals resolved by leaf rank. A leaf's box (and so each of its ancestors', which contain
+// it) is never pruned while its mindist, as computed, is at most the square of its distance
+// d, as computed. Exactly, the inflation keeps the box 1e-3 nearer than the element. With u
+// = 2^-24, every coordinate (also the query's) at most M, the rounding can take away at most
+//   box corner u M, mindist 2 u d, d and its square 3.5 u d, and for a segment the closest
+//   point on it sqrt(2) u M + 2 u |segment| <= 7.1 u M
+// so 8.1 u M + 5.5 u d < 1e-3 suffices for segments, u M + 5.5 u d < 1e-3 for vertices (1e-3
+// / u = 16777): M to 1,700 and 8,000. Beyond (a scene at 1e5 from the origin, or a query as
+// far from it, where two segments of one vertex tie as a rule) the query replays the
+// reference's order. Near-first against that: 180,000 segments, 200k queries, nearest 0.18 /
+// 2.26 ms, silhouettes 0.49 / 46.8 ms.
+constexpr float kMarginUlps = 16000.0f, kNearestUlps = 9.0f, kSilhouetteUlps = 2.0f, kDistanceUlps = 6.0f;
+// what the coordinates (root box b, which holds them all, and p) take of the margin
+SNCH_DEV float coordinate_ulps(float4 b, float2 p, float per_unit)
+{
+    return per_unit * fmaxf(fmaxf(fmaxf(fabsf(b.x), fabsf(b.y)), fmaxf(fabsf(b.z), fabsf(b.w))),
+                            fmaxf(fabsf(p.x), fabsf(p.y)));
+}
+// an answer at distance d found near-first is the reference's
+SNCH_DEV bool settled2(float used, float d) { return used + kDistanceUlps * d <= kMarginUlps; }
+
 SNCH_DEV void leaf_nearest2(const Tree2 &t, uint32_t pos, uint32_t rank, float2 p, float &best, uint32_t &best_rank,
                             uint32_t &best_pos)
 {
@@ -567,6 +588,71 @@ SNCH_DEV void leaf_nearest2(const Tree2 &t, uint32_t pos, uint32_t rank, float2 
         best_pos = pos;
     }
 }
+// The reference's order (query.cuh:239-318), one lane; t.n > 1. A call of its own, so that
+// the near-first searches keep their registers.
+struct Found2
+{
+    float best;   // nearest: squared distance; silhouette: distance
+    uint32_t id;  // sorted position of the segment; silhouette: vertex
+};
+__device__ __noinline__ Found2 nearest2_in_order(Tree2 t, float2 p)
+{
+    const uint32_t ni = t.n - 1;
+    uint32_t sn[kStackDepth];
+    float sd[kStackDepth];
+    Found2 f{INFINITY, kInvalid};
+    int sp = 0;
+    sn[sp] = 0;
+    sd[sp++] = mindist2(node_box2(t, 0), p);
+    while (sp > 0)
+    {
+        --sp;
+        if (sd[sp] > f.best)
+            continue;
+        const Inner2 *rec = t.inner + sn[sp];
+        const B2 lb = unpack_b2(__ldg(&rec->lb)), rb = unpack_b2(__ldg(&rec->rb));
+        const uint4 ch = __ldg(&rec->ch);
+        const float Lmd = mindist2(lb, p), Rmd = mindist2(rb, p);
+        const bool aL = Lmd <= minmaxdist2(rb, p), aR = Rmd <= minmaxdist2(lb, p);
+        for (int k = 0; k < 2; ++k)
+        {
+            if (!(k ? aR : aL))
+                continue;
+            const uint32_t child = k ? ch.y : ch.x;
+            if (child >= ni)
+            {
+                const float4 g = __ldg(t.leaf_seg + (child - ni));
+                float d = sqrtf(closest_point_segment2_sq(f2(g.x, g.y), f2(g.z, g.w), p));
+                d *= d;
+                if (d <= f.best)
+                    f = Found2{d, child - ni};
+                continue;
+            }
+            if (sp >= kStackDepth)
+            {
+                atomicOr(t.status, kStatusStackOverflow);
+                return Found2{NAN, kInvalid};
+            }
+            sn[sp] = child;
+            sd[sp++] = k ? Rmd : Lmd;
+        }
+    }
+    return f;
+}
+// what a nearest query of this point takes of the margin; unsettled from the start if the
+// coordinates, or the distance to the scene, take all of it (or for a NaN point)
+SNCH_DEV float nearest2_ulps(const Tree2 &t, float2 p)
+{
+    const float4 b = __ldg(t.aabbs);
+    const float used = coordinate_ulps(b, p, kNearestUlps);
+    return settled2(used, sqrtf(mindist2(unpack_b2(b), p))) ? used : INFINITY;
+}
+SNCH_DEV void store_nearest2(const Tree2 &t, int64_t q, float best, uint32_t pos, uint32_t *__restrict__ out_idx,
+                             float *__restrict__ out_dist)
+{
+    out_idx[q] = pos == kInvalid ? kInvalid : __ldg(t.order + pos);
+    out_dist[q] = sqrtf(best);
+}
 __global__ void __launch_bounds__(128) nearest2_kernel(Tree2 t, const float *__restrict__ pts, int64_t n,
                                                        uint32_t *__restrict__ out_idx, float *__restrict__ out_dist)
 {
@@ -577,9 +663,10 @@ __global__ void __launch_bounds__(128) nearest2_kernel(Tree2 t, const float *__r
     uint32_t best_pos = kInvalid, best_rank = 0;
     float best = INFINITY;
     const uint32_t ni = t.n - 1;
+    const float used = t.n > 1 ? nearest2_ulps(t, p) : 0.0f;
     if (t.n == 1)
         leaf_nearest2(t, 0u, 0u, p, best, best_rank, best_pos);
-    else if (t.n > 1)
+    else if (t.n > 1 && used < INFINITY)
     {
         uint32_t sn[kStackDepth];
         float sd[kStackDepth];
@@ -633,8 +720,13 @@ __global__ void __launch_bounds__(128) nearest2_kernel(Tree2 t, const float *__r
             }
         }
     }
-    out_idx[q] = best_pos == kInvalid ? kInvalid : __ldg(t.order + best_pos);
-    out_dist[q] = sqrtf(best);
+    if (t.n > 1 && (used == INFINITY || (best_pos != kInvalid && !settled2(used, sqrtf(best)))))
+    {
+        const Found2 f = nearest2_in_order(t, p);
+        best = f.best;
+        best_pos = f.id;
+    }
+    store_nearest2(t, q, best, best_pos, out_idx, out_dist);
 }
 
 // is_silhouette_vertex scene.cuh:112-141
@@ -717,11 +809,76 @@ SNCH_DEV bool cone_test2(const C2 &bc, float2 o, const B2 &b, float dist_to_box)
                               __fmaf_rn(bc.axis.x, v.x, bc.axis.y * v.y));
     return f >= 0 ? f == 1 : cone_overlap2(bc, o, b, dist_to_box);
 }
-// query_device(nearest_silhouette) query.cuh:326-423 over segments, near-first (as
-// nearest2_kernel: the cone tests alone decide which leaves can be reached); also the
-// silhouette vertex (mesh vertex id) of the answer. 180,000 segments, 200k queries
-// 46.8 -> 0.49 ms. kDefer: a query that is not done after kLaneTurns2 expansions is left
-// to the next launch.
+// The reference's order (query.cuh:326-423), one lane; t.n > 1
+__device__ __noinline__ Found2 silhouette2_in_order(Tree2 t, float2 p, bool flip)
+{
+    const uint32_t ni = t.n - 1;
+    uint32_t sn[kStackDepth];
+    float sd[kStackDepth];
+    Found2 f{INFINITY, (uint32_t)-1};
+    int sp = 0;
+    sn[sp] = 0;
+    sd[sp++] = mindist2(node_box2(t, 0), p);
+    while (sp > 0)
+    {
+        --sp;
+        if (sd[sp] > f.best * f.best)
+            continue;
+        const uint32_t node = sn[sp];
+        const uint4 ch = __ldg(&t.inner[node].ch);
+        for (int k = 0; k < 2; ++k)
+        {
+            const B2 b = unpack_b2(__ldg(k ? &t.inner[node].rb : &t.inner[node].lb));
+            const C2 c = unpack_c2(__ldg(k ? &t.inner_cones[node].r : &t.inner_cones[node].l));
+            const float md = mindist2(b, p);
+            if (!(c.half_angle >= 0.0f && cone_overlap2(c, p, b, md)))
+                continue;
+            const uint32_t child = k ? ch.y : ch.x;
+            if (child >= ni)
+            {
+                // the owned vertices in turn, by the squared bound of the leaf so far
+                float bound = f.best * f.best, d = INFINITY;
+                uint32_t id = f.id;
+                bool found = false;
+                for (uint32_t e = 0; e < (k ? ch.w : ch.z) >> 30 && bound > 0.0f; ++e)
+                {
+                    const Vert2 *r = t.leaf_verts + 2 * (uint64_t)(child - ni) + e;
+                    const float4 va = __ldg(&r->a), vb = __ldg(&r->b);
+                    const float2 vd = f2(p.x - va.x, p.y - va.y);
+                    const float l = len2(vd);
+                    if (l * l <= bound && (__float_as_uint(vb.z) != 3u ||
+                                           is_silhouette_vertex(f2(va.z, va.w), f2(vb.x, vb.y), vd, l, flip)))
+                    {
+                        d = l;
+                        bound = l * l;
+                        id = __float_as_uint(vb.w);
+                        found = true;
+                    }
+                }
+                if (found && d <= f.best)
+                    f = Found2{d, id};
+                continue;
+            }
+            if (sp >= kStackDepth)
+            {
+                atomicOr(t.status, kStatusStackOverflow);
+                return Found2{NAN, (uint32_t)-1};
+            }
+            sn[sp] = child;
+            sd[sp++] = md;
+        }
+    }
+    return f;
+}
+SNCH_DEV float silhouette2_ulps(const Tree2 &t, float2 p)  // as nearest2_ulps
+{
+    const float4 b = __ldg(t.aabbs);
+    const float used = coordinate_ulps(b, p, kSilhouetteUlps);
+    return settled2(used, sqrtf(mindist2(unpack_b2(b), p))) ? used : INFINITY;
+}
+// query_device(nearest_silhouette) query.cuh:326-423 over segments, near-first; also the
+// silhouette vertex (mesh vertex id) of the answer. kDefer: a query that is not done after
+// kLaneTurns2 expansions is left to the next launch.
 constexpr uint32_t kLaneTurns2 = 64;  // 48: 160,000 queries 389 -> 460 us; 96 the same
 template <bool kDefer>
 __global__ void __launch_bounds__(128) silhouette2_kernel(Tree2 t, const float *__restrict__ pts,
@@ -893,18 +1050,33 @@ SNCH_DEV bool nearest2_coop(const Tree2 &t, float2 p, float &best, uint32_t &bes
     }
     return true;
 }
+// The first lane_blocks blocks: a lane per query, for those that replay the reference's
+// order, which gains nothing from a warp.
 __global__ void __launch_bounds__(32 * kCoopWarps, 16)
     nearest2_coop_kernel(Tree2 t, const float *__restrict__ pts, int64_t n, uint32_t *__restrict__ out_idx,
-                         float *__restrict__ out_dist)
+                         float *__restrict__ out_dist, unsigned lane_blocks)
 {
     __shared__ CoopStack s_stack[kCoopWarps];
+    if (blockIdx.x < lane_blocks)
+    {
+        const int64_t q = blockIdx.x * (int64_t)(32 * kCoopWarps) + threadIdx.x;
+        if (q >= n)
+            return;
+        const float2 p = load_pt2(pts, q);
+        if (nearest2_ulps(t, p) < INFINITY)
+            return;
+        const Found2 f = nearest2_in_order(t, p);
+        store_nearest2(t, q, f.best, f.id, out_idx, out_dist);
+        return;
+    }
     const int w = threadIdx.x >> 5;
-    const int64_t q = blockIdx.x * (int64_t)kCoopWarps + w;
+    const int64_t q = (blockIdx.x - lane_blocks) * (int64_t)kCoopWarps + w;
     if (q >= n)
         return;
+    const float2 p = load_pt2(pts, q);
     float best = INFINITY;
     uint32_t best_rank = 0, best_pos = kInvalid;
-    if (!nearest2_coop(t, load_pt2(pts, q), best, best_rank, best_pos, s_stack[w]))
+    if (!nearest2_coop(t, p, best, best_rank, best_pos, s_stack[w]))
     {
         if ((threadIdx.x & 31) == 0)
             atomicOr(t.status, kStatusStackOverflow);
@@ -913,8 +1085,16 @@ __global__ void __launch_bounds__(32 * kCoopWarps, 16)
     }
     if ((threadIdx.x & 31) != 0)
         return;
-    out_idx[q] = best_pos == kInvalid ? kInvalid : __ldg(t.order + best_pos);
-    out_dist[q] = sqrtf(best);
+    const float used = nearest2_ulps(t, p);
+    if (used == INFINITY)
+        return;
+    if (best_pos != kInvalid && !settled2(used, sqrtf(best)))
+    {
+        const Found2 f = nearest2_in_order(t, p);
+        best = f.best;
+        best_pos = f.id;
+    }
+    store_nearest2(t, q, best, best_pos, out_idx, out_dist);
 }
 
 SNCH_DEV bool silhouette2_coop(const Tree2 &t, float2 p, bool flip, float &best, uint32_t &best_key, int32_t &best_vert,
@@ -989,12 +1169,15 @@ SNCH_DEV bool silhouette2_coop(const Tree2 &t, float2 p, bool flip, float &best,
     }
     return true;
 }
+// kSettle: the answer is settled here (silhouette2_coop_kernel), not by the pass after
+template <bool kSettle>
 SNCH_DEV void silhouette2_coop_query(const Tree2 &t, const float *__restrict__ pts, const uint8_t *__restrict__ flips,
                                      float *__restrict__ out_dist, int32_t *__restrict__ out_vid, int64_t q, float best,
                                      uint32_t best_key, int32_t best_vert, CoopStack &s)
 {
     const bool flip = flips ? __ldg(flips + q) != 0 : false;
-    if (!silhouette2_coop(t, load_pt2(pts, q), flip, best, best_key, best_vert, s))
+    const float2 p = load_pt2(pts, q);
+    if (!silhouette2_coop(t, p, flip, best, best_key, best_vert, s))
     {
         if ((threadIdx.x & 31) == 0)
             atomicOr(t.status, kStatusStackOverflow);
@@ -1003,19 +1186,45 @@ SNCH_DEV void silhouette2_coop_query(const Tree2 &t, const float *__restrict__ p
     }
     if ((threadIdx.x & 31) != 0)
         return;
+    if (kSettle)
+    {
+        const float used = silhouette2_ulps(t, p);
+        if (used == INFINITY)
+            return;  // replayed by a lane of its own
+        if (best_vert >= 0 && !settled2(used, best))
+        {
+            const Found2 f = silhouette2_in_order(t, p, flip);
+            best = f.best;
+            best_vert = (int32_t)f.id;
+        }
+    }
     out_dist[q] = best;
     if (out_vid)
         out_vid[q] = best_vert;
 }
 __global__ void __launch_bounds__(32 * kCoopWarps, 16)
     silhouette2_coop_kernel(Tree2 t, const float *__restrict__ pts, const uint8_t *__restrict__ flips, int64_t n,
-                            float *__restrict__ out_dist, int32_t *__restrict__ out_vid)
+                            float *__restrict__ out_dist, int32_t *__restrict__ out_vid, unsigned lane_blocks)
 {
     __shared__ CoopStack s_stack[kCoopWarps];
+    if (blockIdx.x < lane_blocks)  // as nearest2_coop_kernel
+    {
+        const int64_t q = blockIdx.x * (int64_t)(32 * kCoopWarps) + threadIdx.x;
+        if (q >= n)
+            return;
+        const float2 p = load_pt2(pts, q);
+        if (silhouette2_ulps(t, p) < INFINITY)
+            return;
+        const Found2 f = silhouette2_in_order(t, p, flips ? __ldg(flips + q) != 0 : false);
+        out_dist[q] = f.best;
+        if (out_vid)
+            out_vid[q] = (int32_t)f.id;
+        return;
+    }
     const int w = threadIdx.x >> 5;
-    const int64_t q = blockIdx.x * (int64_t)kCoopWarps + w;
+    const int64_t q = (blockIdx.x - lane_blocks) * (int64_t)kCoopWarps + w;
     if (q < n)
-        silhouette2_coop_query(t, pts, flips, out_dist, out_vid, q, INFINITY, 0u, -1, s_stack[w]);
+        silhouette2_coop_query<true>(t, pts, flips, out_dist, out_vid, q, INFINITY, 0u, -1, s_stack[w]);
 }
 __global__ void __launch_bounds__(32 * kCoopWarps, 16)
     silhouette2_finish_kernel(Tree2 t, const float *__restrict__ pts, const uint8_t *__restrict__ flips,
@@ -1024,8 +1233,29 @@ __global__ void __launch_bounds__(32 * kCoopWarps, 16)
     __shared__ CoopStack s_stack[kCoopWarps];
     uint4 e;
     while (take_deferred(d, e))
-        silhouette2_coop_query(t, pts, flips, out_dist, out_vid, (int64_t)e.x, __uint_as_float(e.y), e.z, (int32_t)e.w,
-                               s_stack[threadIdx.x >> 5]);
+        silhouette2_coop_query<false>(t, pts, flips, out_dist, out_vid, (int64_t)e.x, __uint_as_float(e.y), e.z,
+                                      (int32_t)e.w, s_stack[threadIdx.x >> 5]);
+}
+
+// After the lanes' silhouette searches: the queries that are not settled, a lane each. (The
+// call in the search's own kernel took it from 48 registers to 54, 200k queries 481 -> 559 us;
+// this pass takes 4 us.)
+__global__ void __launch_bounds__(128) silhouette2_settle_kernel(Tree2 t, const float *__restrict__ pts,
+                                                                 const uint8_t *__restrict__ flips, int64_t n,
+                                                                 float *__restrict__ out_dist,
+                                                                 int32_t *__restrict__ out_vid)
+{
+    const int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (q >= n)
+        return;
+    const float2 p = load_pt2(pts, q);
+    const float d = out_dist[q];  // infinite: none found, so nothing was pruned
+    if (settled2(coordinate_ulps(__ldg(t.aabbs), p, kSilhouetteUlps), d < INFINITY ? d : 0.0f))
+        return;
+    const Found2 f = silhouette2_in_order(t, p, flips ? __ldg(flips + q) != 0 : false);
+    out_dist[q] = f.best;
+    if (out_vid)
+        out_vid[q] = (int32_t)f.id;
 }
 
 // intersects_d(ray<float,2>) aabb.cuh:366-390
@@ -1557,7 +1787,10 @@ int snch_scene2_query_nearest(snch_scene2_t s, const float *pts, int64_t n, uint
     const Tree2 t = s->tree();
     cudaStream_t st = S2(stream);
     if (t.n > 1 && n <= kCoopDirect2)
-        nearest2_coop_kernel<<<blocks(n, kCoopWarps), 32 * kCoopWarps, 0, st>>>(t, pts, n, idx, dist);
+    {
+        const unsigned lanes = blocks(n, 32 * kCoopWarps);
+        nearest2_coop_kernel<<<lanes + blocks(n, kCoopWarps), 32 * kCoopWarps, 0, st>>>(t, pts, n, idx, dist, lanes);
+    }
     else
         nearest2_kernel<<<blocks(n, 128), 128, 0, st>>>(t, pts, n, idx, dist);
     note_launch();
@@ -1583,12 +1816,26 @@ int snch_scene2_query_silhouette(snch_scene2_t s, const float *pts, const uint8_
             [&](const DeferArgs &d, unsigned g) {
                 silhouette2_finish_kernel<<<g, 32 * kCoopWarps, 0, st>>>(t, pts, flip, dist, vertex, d);
             }));
+        silhouette2_settle_kernel<<<blocks(n, 128), 128, 0, st>>>(t, pts, flip, n, dist, vertex);
+        note_launch();
+        SNCH2_CUDA(cudaGetLastError());
         return SNCH_OK;
     }
     if (t.n > 1 && n <= kCoopDirect2)
-        silhouette2_coop_kernel<<<blocks(n, kCoopWarps), 32 * kCoopWarps, 0, st>>>(t, pts, flip, n, dist, vertex);
+    {
+        const unsigned lanes = blocks(n, 32 * kCoopWarps);
+        silhouette2_coop_kernel<<<lanes + blocks(n, kCoopWarps), 32 * kCoopWarps, 0, st>>>(t, pts, flip, n, dist,
+                                                                                          vertex, lanes);
+    }
     else
+    {
         silhouette2_kernel<false><<<blocks(n, 128), 128, 0, st>>>(t, pts, flip, n, dist, vertex, DeferArgs());
+        if (t.n > 1)
+        {
+            silhouette2_settle_kernel<<<blocks(n, 128), 128, 0, st>>>(t, pts, flip, n, dist, vertex);
+            note_launch();
+        }
+    }
     note_launch();
     SNCH2_CUDA(cudaGetLastError());
     return SNCH_OK;
