@@ -451,23 +451,29 @@ int snch_batch_query_silhouette_seeded(snch_scene_t scene, const int32_t *mesh, 
  * threads per block, SNCH_OPT_PACKET, SNCH_OPT_PERSISTENT) = (2, 128, 1, 0)
  * [warp packets: 32 queries per traversal], (2, 128, 0, 0), (4, 128, 0, 0),
  * (8, 128, 0, 0), (2, 64, 0, 0), (2, 256, 0, 0) [one query per traversal],
- * (2, 128, 0, 1) [persistent work-stealing lanes] -- on caller sample batches
+ * (2, 128, 0, 1) [persistent work-stealing lanes] -- and in (2, 128, 2, 0), the
+ * library's own choice by batch size (SNCH_OPT_PACKET 2), on caller sample batches
  * (DEVICE buffers; for a batched scene near_mesh / sil_mesh give each query's
  * mesh, else NULL; a count of 0 skips that query type), keeps the fastest
  * configuration per query type (SNCH_OPT_NODE_WIDTH_*, SNCH_OPT_BLOCK_*,
  * SNCH_OPT_PACKET_*, SNCH_OPT_PERSISTENT_*) and releases the wide records no
- * type keeps. out_ms (HOST, may be NULL): 2 x SNCH_AUTOTUNE_CONFIGS floats,
- * milliseconds per batch in that order for nearest, then silhouette.
- * Synchronous. Distances are the same in every configuration (indices too, up
- * to the exact ties described under SNCH_OPT_PACKET); only their speed
- * differs. Stack depth is not a candidate: a search touches its stack only to
- * the depth it reaches. Give a sample with the query density of the real
- * batches (for a batched scene, all queries of some meshes rather than a few
+ * type keeps. out_ms (HOST, may be NULL): milliseconds per batch in that order
+ * for nearest, then silhouette: snch_autotune writes 2 x SNCH_AUTOTUNE_CONFIGS floats
+ * (without the library's own choice, which it times and may keep all the same),
+ * snch_autotune_all 2 x SNCH_AUTOTUNE_ALL_CONFIGS. Synchronous. Distances are the
+ * same in every configuration (indices too, up to the exact ties described under
+ * SNCH_OPT_PACKET); only their speed differs. Stack depth is not a candidate: a search
+ * touches its stack only to the depth it reaches. Give a sample with the query density
+ * of the real batches (for a batched scene, all queries of some meshes rather than a few
  * of every mesh's): warp packets gain with density and lose on sparse batches. */
 #define SNCH_AUTOTUNE_CONFIGS 7
 int snch_autotune(snch_scene_t scene, const int32_t *near_mesh, const float *near_points, int64_t n_near,
                   const int32_t *sil_mesh, const float *sil_points, const uint8_t *sil_flip_or_null, int64_t n_sil,
                   float *out_ms, snch_stream_t stream);
+#define SNCH_AUTOTUNE_ALL_CONFIGS 8
+int snch_autotune_all(snch_scene_t scene, const int32_t *near_mesh, const float *near_points, int64_t n_near,
+                      const int32_t *sil_mesh, const float *sil_points, const uint8_t *sil_flip_or_null, int64_t n_sil,
+                      float *out_ms, snch_stream_t stream);
 /* node width and threads per block of the nearest (which = 0) or silhouette (1)
  * search; either output may be NULL */
 int snch_get_search_config(snch_scene_t scene, int which, int32_t *out_width, int32_t *out_block);

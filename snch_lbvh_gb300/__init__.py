@@ -292,9 +292,9 @@ class Scene:
         return self.search_config(which)[0]
 
     # (node width, threads per block, OPT_PACKET, OPT_PERSISTENT): warp packets, one query
-    # per traversal, persistent work-stealing lanes
+    # per traversal, persistent work-stealing lanes, the library's own choice by batch size
     AUTOTUNE_CONFIGS = ((2, 128, 1, 0), (2, 128, 0, 0), (4, 128, 0, 0), (8, 128, 0, 0), (2, 64, 0, 0),
-                        (2, 256, 0, 0), (2, 128, 0, 1))
+                        (2, 256, 0, 0), (2, 128, 0, 1), (2, 128, 2, 0))
 
     def autotune(self, near_points=None, sil_points=None, sil_flip=None, near_mesh=None, sil_mesh=None,
                  stream=None):
@@ -310,9 +310,9 @@ class Scene:
         ms_ = None if sil_mesh is None else _dev(sil_mesh, torch.int32)
         k = len(self.AUTOTUNE_CONFIGS)
         out = (C.c_float * (2 * k))()
-        check(lib().snch_autotune(self._h, _ptr(mn), _ptr(pn), 0 if pn is None else pn.shape[0], _ptr(ms_), _ptr(ps),
-                                  _ptr(f), 0 if ps is None else ps.shape[0], C.cast(out, C.c_void_p),
-                                  _stream(stream)))
+        check(lib().snch_autotune_all(self._h, _ptr(mn), _ptr(pn), 0 if pn is None else pn.shape[0], _ptr(ms_),
+                                      _ptr(ps), _ptr(f), 0 if ps is None else ps.shape[0], C.cast(out, C.c_void_p),
+                                      _stream(stream)))
         return {"nearest": dict(zip(self.AUTOTUNE_CONFIGS, out[0:k])),
                 "silhouette": dict(zip(self.AUTOTUNE_CONFIGS, out[k:2 * k]))}
 

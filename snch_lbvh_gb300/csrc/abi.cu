@@ -2007,9 +2007,9 @@ int snch_batch_query_silhouette_seeded(snch_scene_t s, const int32_t *mesh, cons
         reinterpret_cast<const uint32_t *>(mesh));
 }
 
-int snch_autotune(snch_scene_t s, const int32_t *near_mesh, const float *near_pts, int64_t n_near,
-                  const int32_t *sil_mesh, const float *sil_pts, const uint8_t *sil_flip, int64_t n_sil, float *out_ms,
-                  snch_stream_t stream)
+static int autotune(snch_scene_t s, const int32_t *near_mesh, const float *near_pts, int64_t n_near,
+                    const int32_t *sil_mesh, const float *sil_pts, const uint8_t *sil_flip, int64_t n_sil,
+                    float *out_ms, int out_configs, snch_stream_t stream)
 {
     int rc = check_built(s);
     if (rc == SNCH_OK)
@@ -2022,12 +2022,14 @@ int snch_autotune(snch_scene_t s, const int32_t *near_mesh, const float *near_pt
         return rc;
     cudaStream_t st = S(stream);
     // candidates (node width, threads per block, SNCH_OPT_PACKET, SNCH_OPT_PERSISTENT):
-    // warp packets (1: whatever the sample's size), one search per lane, or
-    // persistent work-stealing lanes; the block size applies to the per-lane
+    // warp packets (1: whatever the sample's size), one search per lane,
+    // persistent work-stealing lanes, or the library's own choice by size, which no
+    // fixed form can stand in for (20,011 silhouette queries inside a 20,480-triangle
+    // sphere: 0.9 ms, the fixed forms 10 ms); the block size applies to the per-lane
     // binary searches
-    constexpr int kConfigs = SNCH_AUTOTUNE_CONFIGS;
-    const int cw[kConfigs] = {2, 2, 4, 8, 2, 2, 2}, cb[kConfigs] = {128, 128, 128, 128, 64, 256, 128},
-              cp[kConfigs] = {1, 0, 0, 0, 0, 0, 0}, cr[kConfigs] = {0, 0, 0, 0, 0, 0, 1};
+    constexpr int kConfigs = SNCH_AUTOTUNE_ALL_CONFIGS;
+    const int cw[kConfigs] = {2, 2, 4, 8, 2, 2, 2, 2}, cb[kConfigs] = {128, 128, 128, 128, 64, 256, 128, 128},
+              cp[kConfigs] = {1, 0, 0, 0, 0, 0, 0, 2}, cr[kConfigs] = {0, 0, 0, 0, 0, 0, 1, 0};
     float ms[2][kConfigs] = {};
     char *out = nullptr;
     const int64_t nmax = std::max<int64_t>(1, std::max(n_near, n_sil));
@@ -2135,9 +2137,25 @@ int snch_autotune(snch_scene_t s, const int32_t *near_mesh, const float *near_pt
     }
     if (out_ms)
         for (int kind = 0; kind < 2; ++kind)
-            for (int c = 0; c < kConfigs; ++c)
-                out_ms[kConfigs * kind + c] = ms[kind][c];
+            for (int c = 0; c < out_configs; ++c)
+                out_ms[out_configs * kind + c] = ms[kind][c];
     return SNCH_OK;
+}
+
+int snch_autotune(snch_scene_t s, const int32_t *near_mesh, const float *near_pts, int64_t n_near,
+                  const int32_t *sil_mesh, const float *sil_pts, const uint8_t *sil_flip, int64_t n_sil, float *out_ms,
+                  snch_stream_t stream)
+{
+    return autotune(s, near_mesh, near_pts, n_near, sil_mesh, sil_pts, sil_flip, n_sil, out_ms, SNCH_AUTOTUNE_CONFIGS,
+                    stream);
+}
+
+int snch_autotune_all(snch_scene_t s, const int32_t *near_mesh, const float *near_pts, int64_t n_near,
+                      const int32_t *sil_mesh, const float *sil_pts, const uint8_t *sil_flip, int64_t n_sil,
+                      float *out_ms, snch_stream_t stream)
+{
+    return autotune(s, near_mesh, near_pts, n_near, sil_mesh, sil_pts, sil_flip, n_sil, out_ms,
+                    SNCH_AUTOTUNE_ALL_CONFIGS, stream);
 }
 
 struct snch_graph_s
