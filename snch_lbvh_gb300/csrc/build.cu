@@ -374,11 +374,11 @@ __global__ void __launch_bounds__(256) karras_kernel(BuildArgs a)
     nodes[ni + idx].object = a.vals[idx];
     if (idx == 0)
         nodes[0].parent = kInvalid;
-    if (a.flags)  // the 3D build: nothing has reached a node yet (refit_top_kernel)
+    if (a.flags)  // nothing has reached a node yet (refit_top_kernel, refit2_kernel)
     {
         if (idx < ni)
             a.flags[idx] = 0;
-        if (idx == 0)
+        if (idx == 0 && a.centroids)  // the 3D build
             reinterpret_cast<uint32_t *>(a.centroids)[2 * (uint64_t)n] = 0;  // RefitScratch::count
     }
     if (a.num_meshes)
@@ -885,13 +885,6 @@ __global__ void __launch_bounds__(B, B == kRefitLeaves ? 6 : 1) refit_kernel(Bui
         scratch.exits[s_exit_base + t] = s_exit[t];
 }
 
-// counts an arrival; releases this thread's writes and acquires those of the arrivals before
-SNCH_DEV uint32_t arrive_acq_rel(uint32_t *p)
-{
-    uint32_t old;
-    asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(old) : "l"(p) : "memory");
-    return old;
-}
 // The first thread to reach a node stops; the second (whose sibling's results are
 // published by the sibling's arrival, or by the end of refit_kernel) merges. Bound by the
 // chain of arrivals and merges, so a thread carries its own node's box and cone up and asks

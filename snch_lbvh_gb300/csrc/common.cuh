@@ -425,6 +425,14 @@ SNCH_DEV float ordered_to_float(uint32_t u)
     return __uint_as_float((u & 0x80000000u) ? (u & 0x7FFFFFFFu) : ~u);
 }
 
+// counts an arrival; releases this thread's writes and acquires those of the arrivals before
+SNCH_DEV uint32_t arrive_acq_rel(uint32_t *p)
+{
+    uint32_t old;
+    asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(old) : "l"(p) : "memory");
+    return old;
+}
+
 // ---------------------------------------------------------- cone test filter
 // The shared part of the fast cone tests (2D and 3D): decides the overlap test of a
 // cone (half angle below 90 degrees) from l2 = |v|^2 and av = axis . v, v the offset
