@@ -147,7 +147,7 @@ __global__ void __launch_bounds__(32 * kCoopWarps, 16)
 {
     __shared__ CoopStack s_stack[kCoopWarps];
     uint4 e;
-    while (take_deferred(d, e))
+    for (uint32_t i = first_deferred(); take_deferred(d, i, e); i = next_deferred(d))
         if (e.x != kInvalid)
             nearest_coop_query(t, pts, out_idx, out_dist, seed, (int64_t)e.x,
                                seed.radius ? __ldg(seed.radius + e.x) : INFINITY, __uint_as_float(e.y), e.z, e.w,
@@ -312,7 +312,8 @@ __global__ void __launch_bounds__(32 * kCoopWarps, 14)
     silhouette_coop_query(t, pts, flips, out_dist, out_edge, seed, q, r0, r0, 0u, -1, s_stack[w], s_items[w]);
 }
 
-__global__ void __launch_bounds__(32 * kCoopWarps, 14)
+// (16 blocks, 64 registers: at 66 only 14 fit, and a finish takes 5 % longer)
+__global__ void __launch_bounds__(32 * kCoopWarps, 16)
     silhouette_finish_kernel(TreeView t, const float *__restrict__ pts, const uint8_t *__restrict__ flips,
                              float *__restrict__ out_dist, int32_t *__restrict__ out_edge, SeedArgs seed, DeferArgs d)
 {
@@ -320,7 +321,7 @@ __global__ void __launch_bounds__(32 * kCoopWarps, 14)
     __shared__ CoopEdges s_items[kCoopWarps];
     const int w = threadIdx.x >> 5;
     uint4 e;
-    while (take_deferred(d, e))
+    for (uint32_t i = first_deferred(); take_deferred(d, i, e); i = next_deferred(d))
         if (e.x != kInvalid)
             silhouette_coop_query(t, pts, flips, out_dist, out_edge, seed, (int64_t)e.x,
                                   seed.radius ? __ldg(seed.radius + e.x) : INFINITY, __uint_as_float(e.y), e.z,

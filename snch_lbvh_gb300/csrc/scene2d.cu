@@ -1251,7 +1251,7 @@ __global__ void __launch_bounds__(32 * kCoopWarps, 16)
 {
     __shared__ CoopStack s_stack[kCoopWarps];
     uint4 e;
-    while (take_deferred(d, e))
+    for (uint32_t i = first_deferred(); take_deferred(d, i, e); i = next_deferred(d))
         silhouette2_coop_query<false>(t, pts, flips, out_dist, out_vid, (int64_t)e.x, __uint_as_float(e.y), e.z,
                                       (int32_t)e.w, s_stack[threadIdx.x >> 5]);
 }
