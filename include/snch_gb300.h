@@ -328,6 +328,14 @@ int snch_set_traversal(snch_scene_t scene, int mode);
  *                             or 2^22 rays take 16 at most (two passes). Queries of one
  *                             cell keep their input order; only the speed changes. */
 #define SNCH_OPT_ORDER_BITS 23
+/*   SNCH_OPT_FINISH_LIST      most entries (16 B each, stream-ordered scratch) of the list of
+ *                             searches that one launch leaves to the next (SNCH_OPT_PACKET
+ *                             2). -1 (default): as many as can be left, n at most; 0: none.
+ *                             With fewer, packets that find the list full search on, and
+ *                             batches that run one query per lane first run one query per
+ *                             warp from the start, as they do without memory for the list.
+ *                             Only the speed changes. */
+#define SNCH_OPT_FINISH_LIST 24
 /*   SNCH_OPT_HOST_CHUNK       queries per chunk of the *_host forms (at most 29 bytes in
  *                             and 17 out per query on each of two streams): chunk i's
  *                             input copy, search and output copy run on stream i % 2, so

@@ -39,6 +39,7 @@ OPT_OUTPUT_SCATTER = 20
 OPT_TOP_LEVELS = 21
 OPT_RAY_ORDER = 22
 OPT_ORDER_BITS = 23
+OPT_FINISH_LIST = 24
 
 
 def _torch():

@@ -118,6 +118,7 @@ struct snch_scene_s
     int64_t packet_persistent_min = int64_t(1) << 19;  // packet batches this large run persistent (rays: 4x)
     int output_scatter = 0;  // ordered batches: results in batch order, then one scatter pass (measured slower)
     int ray_order = 0;       // ray batches ordered by length bucket, then origin
+    int64_t finish_list = -1;  // most entries of the list a launch leaves to the next (-1: as needed)
     int order_bits = 24;     // Morton bits of the query-order key of plain scenes (3 sort passes; faster than 30)
     // top tree levels staged in shared memory by the persistent packet searches:
     // the first 2^levels - 1 of kTopSlots heap slots, gathered after every build
@@ -151,6 +152,7 @@ struct snch_scene_s
         t.packet_persistent_min = packet_persistent_min;
         t.out_batch_order_enabled = output_scatter;
         t.order_bits = order_bits;
+        t.finish_list = finish_list;
         if (top_levels > 0 && num_meshes == 0)
         {
             t.top_inner = top_inner;
@@ -1127,6 +1129,11 @@ int snch_set_option(snch_scene_t s, int option, int64_t value)
         if (value < 12 || value > 30)
             return fail(SNCH_ERR_INVALID_ARGUMENT, "SNCH_OPT_ORDER_BITS must be in [12, 30]");
         s->order_bits = (int)value;
+        return SNCH_OK;
+    case SNCH_OPT_FINISH_LIST:
+        if (value < -1)
+            return fail(SNCH_ERR_INVALID_ARGUMENT, "SNCH_OPT_FINISH_LIST must be >= -1");
+        s->finish_list = value;
         return SNCH_OK;
     case SNCH_OPT_RAY_ORDER:
         if (value != 0 && value != 1)
@@ -2417,6 +2424,7 @@ int snch_get_option(snch_scene_t s, int option, int64_t *value)
     case SNCH_OPT_TOP_LEVELS: *value = s->top_levels; break;
     case SNCH_OPT_RAY_ORDER: *value = s->ray_order; break;
     case SNCH_OPT_ORDER_BITS: *value = s->order_bits; break;
+    case SNCH_OPT_FINISH_LIST: *value = s->finish_list; break;
     default: return fail(SNCH_ERR_INVALID_ARGUMENT, "unknown option " + std::to_string(option));
     }
     return SNCH_OK;

@@ -627,7 +627,7 @@ __global__ void __launch_bounds__(kBlock, 1280 / kBlock) nearest_fast_kernel(Tre
         best = r0 * r0;
     }
     bool deferred = false;
-    uint32_t budget = kDefer && defer.list ? kLaneTurns : !kDefer && seed.cap ? seed.cap : 0xFFFFFFFFu;
+    uint32_t budget = kDefer ? kLaneTurns : seed.cap ? seed.cap : 0xFFFFFFFFu;
     const uint32_t ni = t.num_tris - 1;
     const QueryRoot qr = query_root(t, q);
     if (qr.node == kInvalid)
@@ -860,7 +860,7 @@ __global__ void __launch_bounds__(kBlock, 1152 / kBlock) silhouette_fast_kernel(
     uint32_t best_key = 0;
     int32_t best_edge = -1;
     bool deferred = false;
-    uint32_t budget = kDefer && defer.list ? kLaneTurns : !kDefer && seed.cap ? seed.cap : 0xFFFFFFFFu;
+    uint32_t budget = kDefer ? kLaneTurns : seed.cap ? seed.cap : 0xFFFFFFFFu;
     const uint32_t ni = t.num_tris - 1;
     const QueryRoot qr = query_root(t, q);
     if (qr.node == kInvalid)
@@ -3419,9 +3419,10 @@ cudaError_t launch_persistent(void (*kernel)(KArgs...), int64_t n, cudaStream_t 
 // Persistent packets whose long ones end in a second launch (DeferArgs): kernel
 // takes (args..., defer, counter), finish(list, words, sms) launches the rest. The
 // list holds what can be in flight once the batch is handed out: a packet per
-// warp and a chunk per SM's pool.
+// warp and a chunk per SM's pool (at most `most` entries if that is >= 0).
 template <typename Finish, typename... KArgs, typename... Args>
-cudaError_t launch_deferring(void (*kernel)(KArgs...), int64_t n, cudaStream_t st, Finish finish, Args... args)
+cudaError_t launch_deferring(void (*kernel)(KArgs...), int64_t n, int64_t most, cudaStream_t st, Finish finish,
+                             Args... args)
 {
     unsigned grid = 0, sms = 0;
     cudaError_t e = persistent_grid(kernel, 0, n, grid, sms);
@@ -3430,8 +3431,10 @@ cudaError_t launch_deferring(void (*kernel)(KArgs...), int64_t n, cudaStream_t s
     const int64_t in_flight = 32 * (4 * (int64_t)grid + (int64_t)kPoolChunk * sms);
     DeferArgs d;
     d.capacity = (uint32_t)std::min<int64_t>((n + 31) / 32 * 32, in_flight);
+    if (most >= 0)
+        d.capacity = (uint32_t)std::min<int64_t>(d.capacity, most);
     constexpr size_t head = (kWorkBytes + 8 + 255) / 256 * 256;  // counter, pools, list count, list position
-    char *scratch = optional_scratch(head + 16 * (size_t)d.capacity, st, true);
+    char *scratch = d.capacity ? optional_scratch(head + 16 * (size_t)d.capacity, st, true) : nullptr;
     if (scratch)
         d.list = reinterpret_cast<uint4 *>(scratch + head);
     else if ((e = scratch_alloc_raw(reinterpret_cast<void **>(&scratch), head, st)) != cudaSuccess)
@@ -3454,9 +3457,15 @@ cudaError_t launch_deferring(void (*kernel)(KArgs...), int64_t n, cudaStream_t s
     return e != cudaSuccess ? e : f;
 }
 // One query per lane, whose long ones end in a second launch: launch(d) and finish(d,
-// blocks) enqueue the two; without memory for the list the first one alone, all of it
-template <typename Launch, typename Finish>
-cudaError_t launch_lanes_deferring(int64_t n, cudaStream_t st, bool ordered, Launch launch, Finish finish)
+// blocks) enqueue the two. Without scratch for the list (no memory, or under capture, where
+// an unordered batch allocates nothing) direct() searches a warp each from the start. Neither
+// that nor a lane each is the better one throughout, but a lane each may lose more: captured,
+// 30,000 queries, a lane / a warp each, us: nearest / silhouettes in the volume of a
+// 20,480-triangle sphere 1,729 / 226 and 10,327 / 1,029, on its surface, where every search
+// is short, 56 / 121 and 162 / 228; 2M-triangle scene 465 / 209 and 2,774 / 529.
+template <typename Launch, typename Finish, typename Direct>
+cudaError_t launch_lanes_deferring(int64_t n, int64_t most, cudaStream_t st, bool ordered, Launch launch,
+                                   Finish finish, Direct direct)
 {
     int dev = 0, sms = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -3466,10 +3475,11 @@ cudaError_t launch_lanes_deferring(int64_t n, cudaStream_t st, bool ordered, Lau
         return e;
     DeferArgs d;
     // an ordered batch has scratch in the capture already
-    char *scratch = optional_scratch(256 + 16 * (size_t)n, st, ordered);
+    const bool listed = most < 0 || most >= n;
+    char *scratch = listed ? optional_scratch(256 + 16 * (size_t)n, st, ordered) : nullptr;
     if (!scratch)
     {
-        launch(d);
+        direct();
         note_launch();
         return cudaGetLastError();
     }
@@ -3592,6 +3602,9 @@ cudaError_t launch_nearest(const TreeView &t0, const float *pts, int64_t n, uint
     }
     cudaError_t e = cudaSuccess;
     bool launched = false;
+    const auto direct = [&] {  // a warp per query
+        nearest_coop_kernel<<<grid_for(n, kCoopWarps), 32 * kCoopWarps, 0, st>>>(t, pts, n, idx, dist, seed);
+    };
     if (packets)
     {
         // persistent packets for large batches: the same packets and answers, 2-7 %
@@ -3614,7 +3627,7 @@ cudaError_t launch_nearest(const TreeView &t0, const float *pts, int64_t n, uint
                                       DeferArgs());
             else
                 e = launch_deferring(
-                    nearest_packet_persistent_kernel<false>, n, st,
+                    nearest_packet_persistent_kernel<false>, n, t.finish_list, st,
                     [&](const DeferArgs &d, unsigned blocks) {
                         nearest_finish_kernel<<<blocks, 32 * kCoopWarps, 0, st>>>(t, pts, idx, dist, seed, d);
                     },
@@ -3645,18 +3658,19 @@ cudaError_t launch_nearest(const TreeView &t0, const float *pts, int64_t n, uint
     else if (coop && n > kCoopDirect)
     {
         e = launch_lanes_deferring(
-            n, st, t.order != nullptr,
+            n, t.finish_list, st, t.order != nullptr,
             [&](const DeferArgs &d) {
                 nearest_fast_kernel<false, 128, true><<<grid_for(n, 128), 128, 0, st>>>(t, pts, n, idx, dist, nullptr,
                                                                                        seed, d);
             },
             [&](const DeferArgs &d, unsigned blocks) {
                 nearest_finish_kernel<<<blocks, 32 * kCoopWarps, 0, st>>>(t, pts, idx, dist, seed, d);
-            });
+            },
+            direct);
         launched = true;
     }
     else if (coop)
-        nearest_coop_kernel<<<grid_for(n, kCoopWarps), 32 * kCoopWarps, 0, st>>>(t, pts, n, idx, dist, seed);
+        direct();
     else if (t.near_first && t.block_near == 64)
         nearest_fast_kernel<false, 64><<<grid_for(n, 64), 64, 0, st>>>(t, pts, n, idx, dist, nullptr, seed);
     else if (t.near_first && t.block_near == 256)
@@ -3708,6 +3722,9 @@ cudaError_t launch_silhouette(const TreeView &t0, const float *pts, const uint8_
     }
     cudaError_t e = cudaSuccess;
     bool launched = false;
+    const auto direct = [&] {
+        silhouette_coop_kernel<<<grid_for(n, kCoopWarps), 32 * kCoopWarps, 0, st>>>(t, pts, flip, n, dist, edge, seed);
+    };
     if (packets)
     {
         if (stats)
@@ -3726,7 +3743,7 @@ cudaError_t launch_silhouette(const TreeView &t0, const float *pts, const uint8_
                                       seed, DeferArgs());
             else
                 e = launch_deferring(
-                    silhouette_packet_persistent_kernel<false>, n, st,
+                    silhouette_packet_persistent_kernel<false>, n, t.finish_list, st,
                     [&](const DeferArgs &d, unsigned blocks) {
                         silhouette_finish_kernel<<<blocks, 32 * kCoopWarps, 0, st>>>(t, pts, flip, dist, edge, seed, d);
                     },
@@ -3759,18 +3776,19 @@ cudaError_t launch_silhouette(const TreeView &t0, const float *pts, const uint8_
     else if (coop && n > kCoopDirect)
     {
         e = launch_lanes_deferring(
-            n, st, t.order != nullptr,
+            n, t.finish_list, st, t.order != nullptr,
             [&](const DeferArgs &d) {
                 silhouette_fast_kernel<false, 128, true>
                     <<<grid_for(n, 128), 128, 0, st>>>(t, pts, flip, n, dist, edge, nullptr, seed, d);
             },
             [&](const DeferArgs &d, unsigned blocks) {
                 silhouette_finish_kernel<<<blocks, 32 * kCoopWarps, 0, st>>>(t, pts, flip, dist, edge, seed, d);
-            });
+            },
+            direct);
         launched = true;
     }
     else if (coop)
-        silhouette_coop_kernel<<<grid_for(n, kCoopWarps), 32 * kCoopWarps, 0, st>>>(t, pts, flip, n, dist, edge, seed);
+        direct();
     else if (t.near_first && t.block_sil == 64)
         silhouette_fast_kernel<false, 64><<<grid_for(n, 64), 64, 0, st>>>(t, pts, flip, n, dist, edge, nullptr, seed);
     else if (t.near_first && t.block_sil == 256)

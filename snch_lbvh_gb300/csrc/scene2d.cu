@@ -929,7 +929,7 @@ __global__ void __launch_bounds__(128) silhouette2_kernel(Tree2 t, const float *
         int sp = 0;
         uint32_t node = 0;
         bool live = true;
-        uint32_t turns = kDefer && defer.list ? kLaneTurns2 : 0xFFFFFFFFu;
+        uint32_t turns = kDefer ? kLaneTurns2 : 0xFFFFFFFFu;
         while (live)
         {
             if (kDefer && turns-- == 0)
@@ -1595,9 +1595,10 @@ namespace
 // 460 / 361 (200,000: 516 / 547; nearest with lanes first, 130,000: 179 / 195).
 constexpr int64_t kCoopDirect2 = 24576, kLanesFirst2 = 131072;
 // launch(d): the lanes, finish(d, blocks): the warps that finish their list; without memory
-// for the list, or under capture (no allocation in the graph, as before), the lanes alone
-template <typename Launch, typename Finish>
-cudaError_t launch_lanes_first2(int64_t n, cudaStream_t st, Launch launch, Finish finish)
+// for the list, or under capture (no allocation in the graph), direct(): a warp each (180,000
+// segments, a lane / a warp each: 30,000 queries 2,391 / 320 us, 130,000 2,906 / 1,003)
+template <typename Launch, typename Finish, typename Direct>
+cudaError_t launch_lanes_first2(int64_t n, cudaStream_t st, Launch launch, Finish finish, Direct direct)
 {
     int dev = 0, sms = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -1609,7 +1610,7 @@ cudaError_t launch_lanes_first2(int64_t n, cudaStream_t st, Launch launch, Finis
     char *scratch = optional_scratch(256 + 16 * (size_t)n, st, false);
     if (!scratch)
     {
-        launch(d);
+        direct();
         note_launch();
         return cudaGetLastError();
     }
@@ -1823,6 +1824,15 @@ int snch_scene2_query_silhouette(snch_scene2_t s, const float *pts, const uint8_
         return rc;
     const Tree2 t = s->tree();
     cudaStream_t st = S2(stream);
+    const auto settle = [&] {
+        silhouette2_settle_kernel<<<blocks(n, 128), 128, 0, st>>>(t, pts, flip, n, dist, vertex);
+        note_launch();
+    };
+    const auto direct = [&] {  // a warp per query
+        const unsigned lanes = blocks(n, 32 * kCoopWarps);
+        silhouette2_coop_kernel<<<lanes + blocks(n, kCoopWarps), 32 * kCoopWarps, 0, st>>>(t, pts, flip, n, dist,
+                                                                                          vertex, lanes);
+    };
     if (t.n > 1 && n > kCoopDirect2 && n <= kLanesFirst2)
     {
         SNCH2_CUDA(launch_lanes_first2(
@@ -1832,26 +1842,18 @@ int snch_scene2_query_silhouette(snch_scene2_t s, const float *pts, const uint8_
             },
             [&](const DeferArgs &d, unsigned g) {
                 silhouette2_finish_kernel<<<g, 32 * kCoopWarps, 0, st>>>(t, pts, flip, dist, vertex, d);
-            }));
-        silhouette2_settle_kernel<<<blocks(n, 128), 128, 0, st>>>(t, pts, flip, n, dist, vertex);
-        note_launch();
-        SNCH2_CUDA(cudaGetLastError());
+                settle();
+            },
+            direct));
         return SNCH_OK;
     }
     if (t.n > 1 && n <= kCoopDirect2)
-    {
-        const unsigned lanes = blocks(n, 32 * kCoopWarps);
-        silhouette2_coop_kernel<<<lanes + blocks(n, kCoopWarps), 32 * kCoopWarps, 0, st>>>(t, pts, flip, n, dist,
-                                                                                          vertex, lanes);
-    }
+        direct();
     else
     {
         silhouette2_kernel<false><<<blocks(n, 128), 128, 0, st>>>(t, pts, flip, n, dist, vertex, DeferArgs());
         if (t.n > 1)
-        {
-            silhouette2_settle_kernel<<<blocks(n, 128), 128, 0, st>>>(t, pts, flip, n, dist, vertex);
-            note_launch();
-        }
+            settle();
     }
     note_launch();
     SNCH2_CUDA(cudaGetLastError());
