@@ -3363,6 +3363,12 @@ constexpr int64_t kCoopNearestMax = 98304, kCoopSilhouetteMax = 131072;
 // packets of 32 neighbours reach far (2M-triangle scene, packets / lanes first, ms:
 // 140,000 queries 1.91 / 1.42, 220,000 2.62 / 2.13, 300,000 3.00 / 2.78, 400,000 3.47 / 3.55).
 constexpr int64_t kCoopSilhouetteSparseMax = 1 << 18;
+// Crowded ones, ordered batches of 192 queries per triangle and more, run as packets at any
+// size: such a mesh bounds every search, so lanes and then warps search it twice (320
+// triangles, lanes first / packets, us: 70,000 queries 382 / 187, 131,072 601 / 213, from its
+// surface 518 / 244; 1,280 triangles, 131,072 queries, 102 a triangle: 876 / 480 in its
+// volume, but 288 / 385 from its surface and 955 / 1,396 from afar).
+constexpr uint64_t kPacketCrowdedPerTri = 192;
 // the wide searches serve near-first, one-thread-per-query, uncapped launches
 // over a tree whose wide records of that width exist
 inline bool wide_ok(const TreeView &t, int width, bool persistent, const SeedArgs &seed)
@@ -3701,7 +3707,8 @@ cudaError_t launch_silhouette(const TreeView &t0, const float *pts, const uint8_
         return cudaSuccess;
     TreeView t = t0;
     const bool persistent = (t.persistent & 2) != 0;
-    const bool coop = !stats &&
+    const bool crowded = t.order_coherent && (uint64_t)n >= kPacketCrowdedPerTri * t.num_tris;
+    const bool coop = !stats && !crowded &&
                       n <= (8 * (uint64_t)n <= t.num_tris ? kCoopSilhouetteSparseMax : kCoopSilhouetteMax) &&
                       coop_ok(t, t.packet_sil, t.width_sil, t.block_sil, persistent, seed);
     const bool packets = !coop && packet_ok(t, t.packet_sil, t.width_sil, seed);

@@ -134,3 +134,18 @@ def test_sparse_silhouette_ids(n):
     np.testing.assert_array_equal(bits(d), bits(d0))
     check_edge_ids(e, e0, d0, p, v, s.export_topology()[2])
     assert s.device_status() == 0
+
+
+@pytest.mark.parametrize("n", [320 * 192 - 1, 65_535, 65_536, 131_073])
+def test_crowded_silhouette_batches(n):
+    """Around the size at which an ordered batch of a small mesh runs as packets."""
+    import snch_lbvh_gb300 as snch
+    from snch_lbvh_gb300 import meshes
+    v, f = meshes.noisy_icosphere(2, 1.0, 0.01, seed=0)
+    s = built_scene(snch, v, f)
+    rng = np.random.default_rng(n)
+    p = (rng.random((n, 3)) * 2.4 - 1.2).astype(np.float32)
+    flip = (rng.random(n) < 0.5).astype(np.uint8)
+    got = s.query_nearest(p) + s.query_silhouette(p, flip)
+    s.set_option(snch.OPT_PACKET, 0)
+    compare(s, v, f, p, got, s.query_nearest(p) + s.query_silhouette(p, flip))
