@@ -64,7 +64,8 @@ struct NodeRec
 // its DFS rank | owned-edge count << 30, so the silhouette traversal reaches a leaf's
 // edges without reading its LeafRec; an internal child's says whether its cone test is
 // settled whatever the query (kConePass: half angle of 90 degrees or more, kConeFail: no
-// edges), so that a node whose children are both settled is expanded without its cones.
+// edges), for traversals over the view; the searches here read the cones all the same
+// (silhouette_packet_chunk says why).
 struct alignas(64) InnerRec
 {
     float4 a, b, c, d;

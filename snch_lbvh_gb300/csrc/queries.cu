@@ -806,8 +806,9 @@ SNCH_DEV void edge_record_candidate(const TreeView &t, uint64_t slot, uint32_t k
     bool is_sil = (flags & 1u) == 0u || (flags & 2u) == 0u;
     if (!is_sil)
     {
-        float4 ec, ed;
-        load32(e + 2, ec, ed);
+        // two loads: as one of 32 bytes its eight registers in a row made the per-lane search
+        // spill (20,000 queries of a 5,120-triangle sphere 1.79 -> 1.88 ms)
+        const float4 ec = __ldg(e + 2), ed = __ldg(e + 3);
         is_sil = is_silhouette_edge(pa, pb, mk(ec.x, ec.y, ec.z), mk(ed.x, ed.y, ed.z),
                                     mk(o.x - cp.x, o.y - cp.y, o.z - cp.z), d, flip);
     }
@@ -1922,35 +1923,27 @@ SNCH_DEV void silhouette_packet_chunk(const TreeView &t, const float *__restrict
             {
                 if (kStats)
                     ++n_int;
+                // asked for with the node's record, also where InnerRec says that neither cone
+                // test depends on the query: reading them only after that costs every other
+                // node a round trip (2.4M queries of batched meshes 44.4 / 43.0 ms, 2,000 in
+                // forced packets 4.07 / 3.66 ms; 16M of the 2M-triangle scene 30.91 / 30.94)
+                InnerConeRec icr;
+                if (in_top)
+                    icr = s_topc[slot];
+                else
+                {
+                    const float4 *cr = reinterpret_cast<const float4 *>(t.inner_cones + node);
+                    icr.a = __ldg(cr);
+                    icr.b = __ldg(cr + 1);
+                    icr.c = __ldg(cr + 2);
+                }
+                Cone lc, rc;
+                unpack_cones(icr, lc, rc);
                 Lmd = mindist(lb, p);
                 Rmd = mindist(rb, p);
                 const float b2 = best * best;
-                hitL = Lmd <= b2;
-                hitR = Rmd <= b2;
-                if (L < ni && R < ni && Linfo != 0u && Rinfo != 0u)
-                {
-                    // both cone tests are settled: no cone record is read (a uniform
-                    // branch; 16M queries of the 2M-triangle scene 32.3 -> 31.5 ms)
-                    hitL = hitL && Linfo == kConePass;
-                    hitR = hitR && Rinfo == kConePass;
-                }
-                else
-                {
-                    InnerConeRec icr;
-                    if (in_top)
-                        icr = s_topc[slot];
-                    else
-                    {
-                        const float4 *cr = reinterpret_cast<const float4 *>(t.inner_cones + node);
-                        icr.a = __ldg(cr);
-                        icr.b = __ldg(cr + 1);
-                        icr.c = __ldg(cr + 2);
-                    }
-                    Cone lc, rc;
-                    unpack_cones(icr, lc, rc);
-                    hitL = hitL && lc.half_angle >= 0.0f && cone_test(lc, p, lb, Lmd);
-                    hitR = hitR && rc.half_angle >= 0.0f && cone_test(rc, p, rb, Rmd);
-                }
+                hitL = Lmd <= b2 && lc.half_angle >= 0.0f && cone_test(lc, p, lb, Lmd);
+                hitR = Rmd <= b2 && rc.half_angle >= 0.0f && cone_test(rc, p, rb, Rmd);
                 // the leaf work of both children as one loop of edge_candidate calls
                 // (the left leaf's edges, then the right leaf's, per lane: the order of
                 // two leaf_silhouette_info calls), so a lane with only the right leaf
