@@ -615,6 +615,8 @@ int snch_mlp_predict_radius(snch_mlp_t mlp, const float *points, int64_t n, floa
  * device_counts[3] = {decided and equal, decided and different, left to the
  * exact test}. device_counts[1] must stay 0. */
 int snch_selfcheck_cone_filter(int64_t n, uint64_t seed, uint64_t *device_counts, snch_stream_t stream);
+/* the same for the 2D scenes' cone test */
+int snch_selfcheck_cone_filter2(int64_t n, uint64_t seed, uint64_t *device_counts, snch_stream_t stream);
 
 /* building block: C[M x N] (+)= A[M x K] * B[N x K]^T, bf16 row-major A and B, fp32 C, on
  * tcgen05 with TMA operand loads; M % 128 == 0, K % 64 == 0, N in {64, 128, 192, 256}; all

@@ -497,6 +497,19 @@ SNCH_DEV int cone_filter(float half_angle, float radius, float l2, float av)
     return -1;
 }
 
+// random numbers of the filters' self-checks (splitmix64)
+SNCH_DEV uint64_t check_mix(uint64_t z)
+{
+    z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
+    z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
+    return z ^ (z >> 31);
+}
+SNCH_DEV float unit_rand(uint64_t &st)
+{
+    st += 0x9E3779B97F4A7C15ull;
+    return (float)(check_mix(st) >> 40) * (1.0f / 16777216.0f);
+}
+
 // A candidate whose squared length s exceeds beyond(b) cannot pass a test
 // "sqrtf(s) <= b" (silhouette: b a distance) nor "sqrtf(s)^2 <= b" (nearest: b a
 // squared distance): b (1 + 2^-19), rounded twice, exceeds b (1 + 2^-20), and

@@ -299,18 +299,6 @@ SNCH_DEV bool cone_test(const Cone &bc, f3 o, const Box &b, float dist_to_box)
 // cone_overlap, and where it leaves the decision to cone_overlap, on random
 // boxes, cones and points, half of them placed within 1e-3 rad of the decision
 // boundary. counts[0] agree, counts[1] disagree, counts[2] undecided.
-SNCH_DEV uint64_t mix64(uint64_t z)
-{
-    z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
-    z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
-    return z ^ (z >> 31);
-}
-SNCH_DEV float unit_rand(uint64_t &st)
-{
-    st += 0x9E3779B97F4A7C15ull;
-    return (float)(mix64(st) >> 40) * (1.0f / 16777216.0f);
-}
-
 __global__ void cone_filter_check_kernel(int64_t n, uint64_t seed, unsigned long long *counts)
 {
     __shared__ unsigned long long s_c[3];
@@ -320,7 +308,7 @@ __global__ void cone_filter_check_kernel(int64_t n, uint64_t seed, unsigned long
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i < n)
     {
-        uint64_t st = mix64(seed ^ (0x632BE59BD9B4E019ull * (uint64_t)(i + 1)));
+        uint64_t st = check_mix(seed ^ (0x632BE59BD9B4E019ull * (uint64_t)(i + 1)));
         Box b;
         const f3 c = mk(2.f * unit_rand(st) - 1.f, 2.f * unit_rand(st) - 1.f, 2.f * unit_rand(st) - 1.f);
         const f3 h = mk(exp2f(-12.f + 11.f * unit_rand(st)), exp2f(-12.f + 11.f * unit_rand(st)),

@@ -817,16 +817,57 @@ SNCH_DEV bool cone_overlap2(const C2 &bc, float2 o, const B2 &b, float dist_to_b
     const float hs = bc.half_angle + atan2f(d, s);
     return hs >= kPi2 ? true : (kPi2 >= dax - hs && kPi2 <= dax + hs);
 }
-// the same decision, mostly from the filter (cone_filter)
-SNCH_DEV bool cone_test2(const C2 &bc, float2 o, const B2 &b, float dist_to_box)
+// the same decision from the filter (cone_filter): 1 / 0, -1: left to the exact test
+SNCH_DEV int cone_overlap2_fast(const C2 &bc, float2 o, const B2 &b, float dist_to_box)
 {
     if (bc.half_angle >= kPi2 || dist_to_box < kEps)
-        return true;
+        return 1;
     const float2 c = centroid2(b);
     const float2 v = f2(c.x - o.x, c.y - o.y);
-    const int f = cone_filter(bc.half_angle, bc.radius, __fmaf_rn(v.x, v.x, v.y * v.y),
-                              __fmaf_rn(bc.axis.x, v.x, bc.axis.y * v.y));
+    return cone_filter(bc.half_angle, bc.radius, __fmaf_rn(v.x, v.x, v.y * v.y),
+                       __fmaf_rn(bc.axis.x, v.x, bc.axis.y * v.y));
+}
+SNCH_DEV bool cone_test2(const C2 &bc, float2 o, const B2 &b, float dist_to_box)
+{
+    const int f = cone_overlap2_fast(bc, o, b, dist_to_box);
     return f >= 0 ? f == 1 : cone_overlap2(bc, o, b, dist_to_box);
+}
+// Self-check, as cone_filter_check_kernel: random boxes, cones and points, half of them
+// within 1e-3 rad of the decision. counts[0] agree, [1] disagree, [2] left to the exact test.
+__global__ void cone_filter2_check_kernel(int64_t n, uint64_t seed, unsigned long long *counts)
+{
+    __shared__ unsigned long long s_c[3];
+    if (threadIdx.x < 3)
+        s_c[threadIdx.x] = 0;
+    __syncthreads();
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i < n)
+    {
+        uint64_t st = check_mix(seed ^ (0x632BE59BD9B4E019ull * (uint64_t)(i + 1)));
+        const float2 c = f2(2.f * unit_rand(st) - 1.f, 2.f * unit_rand(st) - 1.f);
+        const float2 h = f2(exp2f(-12.f + 11.f * unit_rand(st)), exp2f(-12.f + 11.f * unit_rand(st)));
+        const B2 b{f2(c.x + h.x, c.y + h.y), f2(c.x - h.x, c.y - h.y)};
+        C2 k;
+        const float ph = 6.2831853f * unit_rand(st);
+        k.axis = f2(cosf(ph), sinf(ph));
+        k.half_angle = unit_rand(st) < 0.5f ? 0.3f * unit_rand(st) : kPi2 * unit_rand(st);
+        k.radius = len2(h) * (0.5f + unit_rand(st));
+        const float l = k.radius * exp2f(-1.f + 6.f * unit_rand(st));
+        // direction at a chosen angle to the axis: random, or near the decision boundary
+        float theta = 6.2831853f * unit_rand(st);
+        if (unit_rand(st) < 0.5f)
+        {
+            const float hs = k.half_angle + (l > k.radius ? asinf(k.radius / l) : 0.f);
+            theta = kPi2 + (unit_rand(st) < 0.5f ? -hs : hs) + 1e-3f * (2.f * unit_rand(st) - 1.f);
+        }
+        const float2 o = f2(c.x - l * cosf(ph + theta), c.y - l * sinf(ph + theta));
+        const float md = mindist2(b, o);
+        const int f = cone_overlap2_fast(k, o, b, md);
+        atomicAdd(&s_c[f < 0 ? 2 : ((f == 1) == cone_overlap2(k, o, b, md) ? 0 : 1)], 1ull);
+    }
+    __syncthreads();
+    if (threadIdx.x < 3 && s_c[threadIdx.x])
+        atomicAdd(counts + threadIdx.x, s_c[threadIdx.x]);
 }
 // The reference's order (query.cuh:326-423), one lane; t.n > 1
 __device__ __noinline__ Found2 silhouette2_in_order(Tree2 t, float2 p, bool flip)
@@ -1904,6 +1945,19 @@ int snch_scene2_sample_on_object(snch_scene2_t s, const int32_t *idx, const floa
     if (rc != SNCH_OK || n == 0)
         return rc;
     sample_point2_kernel<<<blocks(n, 256), 256, 0, S2(stream)>>>(s->verts, s->segs, s->n, idx, u, n, pts);
+    note_launch();
+    SNCH2_CUDA(cudaGetLastError());
+    return SNCH_OK;
+}
+
+int snch_selfcheck_cone_filter2(int64_t n, uint64_t seed, uint64_t *device_counts, snch_stream_t stream)
+{
+    if (n < 0 || !device_counts)
+        return report_error(SNCH_ERR_INVALID_ARGUMENT, "bad count or NULL counts");
+    if (n == 0)
+        return SNCH_OK;
+    cone_filter2_check_kernel<<<blocks(n, 256), 256, 0, S2(stream)>>>(
+        n, seed, reinterpret_cast<unsigned long long *>(device_counts));
     note_launch();
     SNCH2_CUDA(cudaGetLastError());
     return SNCH_OK;

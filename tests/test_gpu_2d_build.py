@@ -34,3 +34,20 @@ def test_tree_and_ranks(oracle_mod, n):
         np.testing.assert_array_equal(bits(dist), bits(od))
         np.testing.assert_array_equal(idx.view(np.uint32), oi)
     assert s.device_status() == 0
+
+
+def test_fast_cone_test_agrees_with_exact():
+    """The 2D cone test's filter decides only where its error bound allows, and then as the
+    exact test: 4M random cases, half of them within 1e-3 rad of the decision."""
+    import ctypes as C
+
+    import snch_lbvh_gb300 as snch
+    import torch
+    counts = torch.zeros(3, dtype=torch.int64, device="cuda")
+    for seed in (1, 2):
+        snch.check(snch.lib().snch_selfcheck_cone_filter2(2_000_000, seed, C.c_void_p(counts.data_ptr()),
+                                                          C.c_void_p(torch.cuda.current_stream().cuda_stream)))
+    agree, disagree, undecided = (int(x) for x in counts.cpu())
+    assert agree + disagree + undecided == 4_000_000
+    assert disagree == 0
+    assert agree >= 0.5 * 4_000_000, (agree, undecided)
