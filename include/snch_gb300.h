@@ -267,13 +267,19 @@ int snch_set_traversal(snch_scene_t scene, int mode);
 /*   SNCH_OPT_PACKET           warp packets for the binary near-first nearest and
  *                             silhouette searches: a warp's 32 queries walk one shared
  *                             traversal, each lane applying its own tests and keeping its
- *                             own answer. 2 (default): the library chooses by size: small
- *                             batches (unordered, or up to 98,304 nearest / 131,072
- *                             silhouette queries) run one query per warp, its 32 lanes
- *                             expanding 32 nodes of that query's search at a time;
- *                             larger ordered batches run as packets (nearest
- *                             batches also need at least 1 query per triangle), whose
- *                             last, long packets finish one query per warp. 1: packets
+ *                             own answer. 2 (default): the library chooses by size.
+ *                             Up to 24,576 queries run one per warp, its 32 lanes
+ *                             expanding 32 nodes of that query's search at a time. Up to
+ *                             98,304 nearest queries (if ordered, at least one per 4
+ *                             triangles) and 131,072 silhouette queries (262,144 with at
+ *                             most one per 8 triangles; ordered ones with 192 or more per
+ *                             triangle not) run one per lane for 32 expansions, and the
+ *                             searches that take longer then one per warp; without
+ *                             memory for their list, or unordered under stream capture,
+ *                             all one per warp. Larger ordered batches run as packets
+ *                             (nearest ones with at least 1 query per triangle), whose
+ *                             last, long packets finish one query per warp; the others
+ *                             run one query per lane. 1: packets
  *                             always; 0: never (each lane walks its own). Same distances;
  *                             the silhouette edge id / nearest index equals the per-lane
  *                             one except on an exact distance tie that falls on a
@@ -294,7 +300,7 @@ int snch_set_traversal(snch_scene_t scene, int mode);
  *                             below 2^20 queries draw packets from the batch's counter
  *                             instead of the pools. */
 #define SNCH_OPT_PACKET_PERSISTENT_MIN 19
-/*   SNCH_OPT_OUTPUT_SCATTER   1: the results of a Morton-ordered, unseeded batch are
+/*   SNCH_OPT_OUTPUT_SCATTER   1: the results of an ordered, unseeded batch are
  *                             written in batch order to a temporary and then moved to
  *                             input order by one scatter pass, so that each warp's stores
  *                             fill whole sectors (written at input positions directly,
@@ -340,7 +346,7 @@ int snch_set_traversal(snch_scene_t scene, int mode);
  *                             and 17 out per query on each of two streams): chunk i's
  *                             input copy, search and output copy run on stream i % 2, so
  *                             copies overlap searches; a larger chunk gives each
- *                             Morton-ordered search a denser batch. 0 (default): 2^24
+ *                             ordered search a denser batch. 0 (default): 2^24
  *                             for nearest / silhouette, 2^22 for ray / sphere sample. */
 #define SNCH_OPT_HOST_CHUNK 15
 int snch_set_option(snch_scene_t scene, int option, int64_t value);

@@ -177,7 +177,7 @@ class Scene:
         check(lib().snch_set_traversal(self._h, int(mode)))
 
     def set_option(self, option: int, value: int):
-        """OPT_TRAVERSAL, OPT_QUERY_ORDER (Morton-sorted batches), OPT_ORDER_MIN_BATCH,
+        """OPT_TRAVERSAL, OPT_QUERY_ORDER (batches sorted along a curve), OPT_ORDER_MIN_BATCH,
         OPT_PERSISTENT, OPT_TAIL_CAP, OPT_NODE_WIDTH[_NEAREST|_SILHOUETTE] (2, 4 or 8)."""
         check(lib().snch_set_option(self._h, int(option), int(value)))
 

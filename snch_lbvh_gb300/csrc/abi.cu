@@ -55,7 +55,7 @@ constexpr size_t kSmallWords = 1056;
 constexpr size_t kWStatus = 1040, kWNumEdges = 1041, kWBad = 1042, kWHist = 8;
 
 // queries per pipelined host-form chunk when SNCH_OPT_HOST_CHUNK is 0 (auto):
-// nearest / silhouette searches gain from a dense Morton-ordered batch, ray and
+// nearest / silhouette searches gain from a dense ordered batch, ray and
 // sphere-sample batches from copies that overlap the next chunk's search
 constexpr int64_t kHostChunkSearch = 1 << 24, kHostChunkRay = 1 << 22;
 
@@ -89,7 +89,7 @@ struct snch_scene_s
     snch_silhouette_edge *ref_edges = nullptr;
     bool topology_ready = false, built = false;
     int traversal = SNCH_TRAVERSAL_NEAR_FIRST;
-    int query_order = 1;             // Morton-sort batches of at least order_min queries
+    int query_order = 1;             // sort batches of at least order_min queries along a curve
     int64_t order_min = 65536;
     int64_t host_chunk = 0;  // queries per pipelined host-form chunk; 0: per query type
     int persistent_near = 0, persistent_sil = 0;  // lane-refill (work-stealing) searches
@@ -114,12 +114,12 @@ struct snch_scene_s
     // and the wide records of the built tree: [0] 4-way, [1] 8-way
     int width_near = 2, width_sil = 2;
     int block_near = 128, block_sil = 128;  // threads per block of the binary searches
-    int packet_near = 2, packet_sil = 2;    // warp packets: 0 never, 1 always, 2 Morton-ordered batches
+    int packet_near = 2, packet_sil = 2;    // warp packets: 0 never, 1 always, 2 by batch size and order
     int64_t packet_persistent_min = int64_t(1) << 19;  // packet batches this large run persistent (rays: 4x)
     int output_scatter = 0;  // ordered batches: results in batch order, then one scatter pass (measured slower)
     int ray_order = 0;       // ray batches ordered by length bucket, then origin
     int64_t finish_list = -1;  // most entries of the list a launch leaves to the next (-1: as needed)
-    int order_bits = 24;     // Morton bits of the query-order key of plain scenes (3 sort passes; faster than 30)
+    int order_bits = 24;     // curve bits of the query-order key of plain scenes (3 sort passes; faster than 30)
     // top tree levels staged in shared memory by the persistent packet searches:
     // the first 2^levels - 1 of kTopSlots heap slots, gathered after every build
     int top_levels = 0;
@@ -635,7 +635,7 @@ int check_n(int64_t n, std::initializer_list<const void *> ptrs)
     return SNCH_OK;
 }
 
-// Tree view for one batch: Morton-sorted query order when enabled (the
+// Tree view for one batch: curve-sorted query order when enabled (the
 // ordering scratch is stream-ordered memory released after the launch).
 struct BatchView
 {
@@ -721,7 +721,7 @@ cudaError_t queue_fallback_count(snch_scene_s *s, int kind, const uint32_t *coun
 }
 
 // One nearest / silhouette batch in up to three passes:
-//   1. the batch (Morton-ordered), seeded with `radius` if given, near-first
+//   1. the batch (ordered), seeded with `radius` if given, near-first
 //      searches capped at tail_cap expansions (the long ones are deferred with
 //      the best distance they had);
 //   2. the deferred queries, seeded with that distance (same results);
@@ -787,7 +787,7 @@ int run_query(snch_scene_s *s, int kind, const float *pts, const float *radius, 
     }
     if (e == cudaSuccess && radius)
     {
-        // The fallback pass runs the failed queries in the batch's own (Morton)
+        // The fallback pass runs the failed queries in the batch's own (curve)
         // order. Failures that cluster (a few percent of a batch, e.g. points
         // far inside a closed mesh) keep neighbouring queries in a warp and run
         // as warp packets; sparse ones (a fraction of a percent spread over the
@@ -1604,7 +1604,7 @@ int snch_query_visits(snch_scene_t s, int kind, const float *in0, const float *i
     char *scratch = nullptr;
     SNCH_CUDA(scratch_alloc(&scratch, 32 * (size_t)n + 256, st));
     // nearest / silhouette batches are counted in the order a query call runs them
-    // (Morton-ordered above the ordering threshold, which selects the packet form)
+    // (ordered above the ordering threshold, which selects the packet form)
     BatchView b;
     cudaError_t e = kind <= 1 ? batch_view(s, in0, n, st, b) : cudaSuccess;
     if (e != cudaSuccess)

@@ -1208,7 +1208,7 @@ cudaError_t launch_build_front(const BuildArgs &a, cudaStream_t st)
     const uint32_t g = (n + 255) / 256;
     leaf_bounds_kernel<<<g, 256, 0, st>>>(a);
     note_launch();
-    morton_kernel<<<std::min(g, 1216u), 256, 0, st>>>(a);
+    morton_kernel<<<std::min(g, kHistogramBlocks), 256, 0, st>>>(a);
     note_launch();
     return cudaGetLastError();
 }

@@ -139,7 +139,7 @@ struct TreeView
     const EdgeRec *edges = nullptr;
     uint32_t *status = nullptr;
     int near_first = 1;               // 1: near-first nearest/silhouette traversal, 0: the reference's stack order
-    const uint32_t *order = nullptr;  // optional: thread i answers query order[i] (Morton-sorted batches)
+    const uint32_t *order = nullptr;  // optional: thread i answers query order[i] (batches sorted along a curve)
     const uint32_t *order_count = nullptr;  // optional: device count of valid entries of order
     int persistent = 0;  // persistent lane-refill kernels (same results): bit 0 nearest, bit 1 silhouette, bit 2 ray
     // batched queries over a batched scene: the mesh of each query (input position)
@@ -155,10 +155,10 @@ struct TreeView
     // threads per block of the binary near-first nearest / silhouette searches (64, 128, 256)
     int block_near = 128, block_sil = 128;
     // warp packets (a warp's 32 queries walk one shared traversal): 0 never,
-    // 1 always, 2 when the batch is Morton-ordered (order_coherent)
+    // 1 always, 2 by batch size where the batch is ordered (order_coherent)
     int packet_near = 0, packet_sil = 0;
     int64_t packet_persistent_min = int64_t(1) << 19;  // packet batches this large run persistent (rays: 4x)
-    int order_coherent = 0;  // order[] is the batch's Morton order (neighbours share warps)
+    int order_coherent = 0;  // order[] follows a curve (neighbours share warps)
     // the internal nodes of the top tree levels in heap order (slot 0 the root,
     // the children of slot i at 2i+1 / 2i+2), staged in shared memory by the
     // persistent packet searches; top_slots = 2^levels - 1, 0 = off
@@ -169,7 +169,7 @@ struct TreeView
     // query order[i]; the launcher then scatters them to query order (unseeded,
     // fully ordered batches of the kernels that support it)
     int64_t finish_list = -1;  // SNCH_OPT_FINISH_LIST
-    int order_bits = 24;  // Morton bits of a plain scene's query-order key (sorted in ceil(bits / 8) passes)
+    int order_bits = 24;  // curve bits of a plain scene's query-order key (sorted in ceil(bits / 8) passes)
     int out_batch_order = 0;
     int out_batch_order_enabled = 0;  // SNCH_OPT_OUTPUT_SCATTER
     const float4 *wide4 = nullptr, *wide8 = nullptr;        // wide records
@@ -294,7 +294,8 @@ SNCH_DEV Box merge_box(const Box &l, const Box &r)
 // a paired product and the paired sum that consumes it into one fused
 // multiply-add despite the explicit rounding modifiers (a GPU probe: 1.6M of
 // 4.2M paired sums of products differed from the scalar ones), which would
-// change the reference's roundings.
+// change the reference's roundings. Paired differences, and paired products whose
+// sums stay scalar, have nothing to fuse; they have not been tried here.
 SNCH_DEV float mindist(const Box &b, f3 p)
 {
     const float dx = fminf(b.upper.x, fmaxf(b.lower.x, p.x)) - p.x;

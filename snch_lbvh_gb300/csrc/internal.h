@@ -138,7 +138,7 @@ cudaError_t launch_sample(const TreeView &t, const float *c, const float *r, con
 // q1 = directions) enumeration: first max_out results per query, total count
 cudaError_t launch_enumerate(const TreeView &t, bool line, const float *q0, const float *q1, int64_t n,
                              uint32_t max_out, uint32_t *idx, float *tt, uint32_t *count, cudaStream_t st);
-// Morton-sorted order of a query batch (thread i answers query order[i]);
+// Order of a query batch along a curve (thread i answers query order[i]);
 // Stream-ordered scratch from the library's memory pool on the current device
 // (kept mapped between calls; cudaMallocAsync under stream capture). Free with
 // cudaFreeAsync on the same stream.
@@ -209,6 +209,9 @@ cudaError_t scan_flags(const uint32_t *in, uint32_t *out, uint32_t n, uint32_t *
 // and the histogram pass is skipped; hist == scratch: the counts were added up at the
 // start of the scratch after clear_sort_scratch.
 constexpr int kSortTile = 4096;
+// Most blocks of the kernels that count digits as they write keys: each flushes 1,024 counts,
+// so as many as are resident at once and no more (8 of 256 threads on each of 152 SMs).
+constexpr unsigned kHistogramBlocks = 8 * 152;
 size_t sort_scratch_bytes(uint32_t n, int key_bits);
 cudaError_t clear_sort_scratch(void *scratch, uint32_t n, int key_bits, cudaStream_t st);
 struct SortResult

@@ -1392,7 +1392,7 @@ __global__ void __launch_bounds__(128, SNCH_WIDE_MIN_BLOCKS)
 
 // ------------------------------------------------------------------ warp packets
 // Packet forms of the near-first nearest / silhouette searches (SNCH_OPT_PACKET):
-// the 32 queries of a warp -- neighbours, when the batch is Morton-ordered --
+// the 32 queries of a warp -- neighbours, when the batch is ordered --
 // walk ONE traversal together. The warp keeps one stack of (node, lane mask)
 // entries in shared memory; at a node every lane whose bit is set applies its
 // own tests to the two children (the record is one broadcast load), the
@@ -1411,7 +1411,7 @@ constexpr int kPacketWarps = 4;  // 128-thread blocks
 // batch) through a pool per SM: a pool holds a chunk of kPoolChunk consecutive
 // packets taken from the batch-wide counter, and the warps of that SM take its
 // packets one at a time, refilling it from the counter when it is used up. At
-// any moment the SMs work on neighbouring chunks of the Morton-ordered batch (a
+// any moment the SMs work on neighbouring chunks of the ordered batch (a
 // window as narrow as with one counter), and the warps of one SM on neighbouring
 // packets, so they also share the tree records in that SM's L1. 16M-query
 // batches of the 2M-triangle scene: nearest 12.04 -> 11.42 ms, silhouette 35.63
@@ -2086,7 +2086,7 @@ __global__ void __launch_bounds__(128, SNCH_SIL_PACKET_MIN_BLOCKS)
 // run the SAME per-query traversal (same visits, same results) but refill a
 // lane with the next query of the batch as soon as its own query finishes:
 // each warp takes chunks of 32 consecutive queries (spatially coherent when
-// the batch is Morton-ordered) from a global counter, and lanes take queries
+// the batch is ordered) from a global counter, and lanes take queries
 // from the warp's chunk in lane order.
 
 struct WarpQueue
@@ -3038,7 +3038,8 @@ SNCH_DEV uint32_t expand_cell(uint32_t v)
     return v;
 }
 // Position of the cell (x, y, z), 10 bits each, on a 3D Hilbert curve of the top
-// `levels` bits (30-bit result, the lower bits 0): J. Skilling, "Programming the
+// `levels` bits: the top 3 x levels of the 30 bits that come back; query_key shifts the
+// others, which have no meaning, out. J. Skilling, "Programming the
 // Hilbert curve", AIP Conf. Proc. 707 (2004), the transposed index, interleaved.
 // Nearest and silhouette batches are ordered along it: a Morton curve jumps, so some
 // packets of 32 consecutive queries spread over far cells and visit the union of their
@@ -3338,11 +3339,19 @@ inline bool coop_ok(const TreeView &t, int packet, int width, int block, bool pe
 // surface, where every search is short, 0.30 / 0.13 and 0.16 / 0.12; 2M-triangle scene,
 // 98,000 queries 1.35 / 1.06. 16 / 64 / 128 expansions: walk on stars, 100,003 walkers,
 // 31.7 / 31.1 / 37.0 ms, 32 28.7.
+// Where every search is short (nearest, from the surface of the queried mesh itself) a lane
+// each alone would be the best form, and the host cannot know: 24,000 such queries, a lane /
+// a warp each, us: 1,280 triangles 36 / 73, 20,480 62 / 104; 65,000, lanes alone / lanes first,
+// 39 / 44, 69 / 82. The same batches in the volume: 468 / 129, 1,665 / 219; 510 / 228, 1,757 /
+// 410. Leaving after 64 expansions instead takes the surface to within 5 % and the volume of
+// the larger meshes 8 to 20 % up.
 constexpr int64_t kCoopDirect = 24576;
 constexpr int64_t kCoopNearestMax = 98304, kCoopSilhouetteMax = 131072;
 // Sparse silhouette batches, at most a query per 8 triangles, keep to it longer: their
 // packets of 32 neighbours reach far (2M-triangle scene, packets / lanes first, ms:
-// 140,000 queries 1.91 / 1.42, 220,000 2.62 / 2.13, 300,000 3.00 / 2.78, 400,000 3.47 / 3.55).
+// 140,000 queries 1.91 / 1.42, 220,000 2.62 / 2.13, 300,000 3.00 / 2.78, 400,000 3.47 / 3.55;
+// tori of 1.3M and 2.2M triangles, 160,000 14.3 / 6.1, 262,144 28.9 / 10.2; a closed sphere of
+// 1.3M, 163,000 144 / 143, from its surface 2.1 / 1.4).
 constexpr int64_t kCoopSilhouetteSparseMax = 1 << 18;
 // Crowded ones, ordered batches of 192 queries per triangle and more, run as packets at any
 // size: such a mesh bounds every search, so lanes and then warps search it twice (320
@@ -3484,7 +3493,7 @@ cudaError_t launch_lanes_deferring(int64_t n, int64_t most, cudaStream_t st, boo
     const cudaError_t f = cudaFreeAsync(scratch, st);
     return e != cudaSuccess ? e : f;
 }
-// Results of an unseeded, fully Morton-ordered batch are written at their batch
+// Results of an unseeded, fully ordered batch are written at their batch
 // position into a stream-ordered temporary (warp-contiguous, coalesced stores)
 // and moved to query order by one scatter pass per batch. Written at query
 // order[i] directly, neighbouring lanes store to unrelated 4-byte slots: each
@@ -3931,7 +3940,7 @@ cudaError_t launch_query_order(const TreeView &t, const float *pts, int64_t n, v
     cudaError_t e = clear_sort_scratch(sort_scratch, (uint32_t)n, sort_bits, st);
     if (e != cudaSuccess)
         return e;
-    query_keys_kernel<<<std::min(grid_for(n, 256), 1216u), 256, 0, st>>>(
+    query_keys_kernel<<<std::min(grid_for(n, 256), kHistogramBlocks), 256, 0, st>>>(
         pts, n, t.aabbs, keys, vals, t, mesh_bits, len, t.query_mesh ? 32 - mesh_bits : code_bits, hilbert,
         sort_passes(sort_bits), sort_scratch);
     note_launch();

@@ -57,6 +57,7 @@ struct Table
     uint32_t stride;  // places per vertex (0: more vertices than slots, hash at once)
 };
 
+// the 64-bit finaliser of MurmurHash3 (A. Appleby, public domain)
 __device__ __forceinline__ unsigned long long mix64(unsigned long long k)
 {
     k ^= k >> 33;
