@@ -655,7 +655,7 @@ def batched_leg(scale, per_tri=8):
     tuned = b.autotune(Pt, Pt, None, near_mesh=Mt, sil_mesh=Mt)
 
     def cfg_name(w, bk, pk, pers):
-        return f"w{w}_b{bk}_" + ("packet" if pk else "persistent" if pers else "lane")
+        return f"w{w}_b{bk}_" + ("auto" if pk == 2 else "packet" if pk else "persistent" if pers else "lane")
 
     chosen = {"near": cfg_name(*b.search_config("nearest")), "sil": cfg_name(*b.search_config("silhouette"))}
     # the full batches again in the chosen configurations
