@@ -9,7 +9,7 @@
 // bit-identical to the reference's; acosf / asinf / atan2f / logf / sinf / cosf
 // are CUDA's. Rays and circle samples replay the reference's traversal order; the
 // nearest and silhouette searches go near-first where that gives its answers, and replay
-// it elsewhere (in_order2).
+// it where it may not (settled2).
 #include <algorithm>
 #include <string>
 
@@ -577,10 +577,17 @@ SNCH_DEV float2 load_pt2(const float *p, int64_t q) { return f2(__ldg(p + 2 * q)
 //   box corner u M, mindist 2 u d, d and its square 3.5 u d, and for a segment the closest
 //   point on it sqrt(2) u M + 2 u |segment| <= 7.1 u M
 // so 8.1 u M + 5.5 u d < 1e-3 suffices for segments, u M + 5.5 u d < 1e-3 for vertices (1e-3
-// / u = 16777): M to 1,700 and 8,000. Beyond (a scene at 1e5 from the origin, or a query as
-// far from it, where two segments of one vertex tie as a rule) the query replays the
-// reference's order. Near-first against that: 180,000 segments, 200k queries, nearest 0.18 /
-// 2.26 ms, silhouettes 0.49 / 46.8 ms.
+// / u = 16777): M to 1,700 and 8,000. Near-first against the reference's order: 180,000
+// segments, 200k queries, nearest 0.18 / 2.26 ms, silhouettes 0.49 / 46.8 ms.
+// Beyond (a scene at 1e5 from the origin, or a query as far from it, where two segments of
+// one vertex tie as a rule) a lane goes near-first once more, pruning only what the same
+// bounds leave no doubt of (reach2): so it sees every leaf at the minimum D. The reference
+// sees such a leaf for certain if its parent's mindist, which it prunes by, is at most D
+// (then so is that of every ancestor, whose box is no smaller, and its best is never below
+// D). If one leaf at D is not certain in that way, the query replays the reference's order.
+// 200k queries of a scene 2,000 across, nearest 195 us (replayed 1,403), of one 8,000 across,
+// silhouettes 1.08 ms (replayed 38 ms); at 1e5 from the origin most warps hold a query that is
+// in doubt: 1.7 and 22 ms.
 constexpr float kMarginUlps = 16000.0f, kNearestUlps = 9.0f, kSilhouetteUlps = 2.0f, kDistanceUlps = 6.0f;
 // what the coordinates (root box b, which holds them all, and p) take of the margin
 SNCH_DEV float coordinate_ulps(float4 b, float2 p, float per_unit)
@@ -590,6 +597,12 @@ SNCH_DEV float coordinate_ulps(float4 b, float2 p, float per_unit)
 }
 // an answer at distance d found near-first is the reference's
 SNCH_DEV bool settled2(float used, float d) { return used + kDistanceUlps * d <= kMarginUlps; }
+// a box at a squared mindist beyond this holds nothing at a distance of d or less
+SNCH_DEV float reach2(float used, float d)
+{
+    const float r = d + (used + kDistanceUlps * d) * 5.9604644775390625e-8f;  // 2^-24
+    return beyond_sq(r * r);
+}
 
 SNCH_DEV void leaf_nearest2(const Tree2 &t, uint32_t pos, uint32_t rank, float2 p, float &best, uint32_t &best_rank,
                             uint32_t &best_pos)
@@ -657,6 +670,74 @@ __device__ __noinline__ Found2 nearest2_in_order(Tree2 t, float2 p)
         }
     }
     return f;
+}
+// A query that is not settled near-first: near-first within reach2, or in the reference's order
+__device__ __noinline__ Found2 nearest2_unsettled(Tree2 t, float2 p)
+{
+    const uint32_t ni = t.n - 1;
+    const float4 root = __ldg(t.aabbs);
+    const float used = coordinate_ulps(root, p, kNearestUlps);
+    uint32_t sn[kStackDepth];
+    float sd[kStackDepth];
+    Found2 f{INFINITY, kInvalid};
+    uint32_t rank = 0, node = 0;
+    float nd = mindist2(unpack_b2(root), p), lim = INFINITY;
+    bool doubt = false;
+    int sp = 0;
+    for (;;)
+    {
+        const Inner2 *rec = t.inner + node;
+        const B2 lb = unpack_b2(__ldg(&rec->lb)), rb = unpack_b2(__ldg(&rec->rb));
+        const uint4 ch = __ldg(&rec->ch);
+        const float md[2] = {mindist2(lb, p), mindist2(rb, p)};
+        const bool ok[2] = {md[0] <= minmaxdist2(rb, p), md[1] <= minmaxdist2(lb, p)};
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+        {
+            const uint32_t child = k ? ch.y : ch.x, info = (k ? ch.w : ch.z) & kLeafRankMask;
+            if (!ok[k] || child < ni || md[k] > lim)
+                continue;
+            const float4 g = __ldg(t.leaf_seg + (child - ni));
+            float d = sqrtf(closest_point_segment2_sq(f2(g.x, g.y), f2(g.z, g.w), p));
+            d *= d;
+            if (!(d <= f.best))
+                continue;
+            const bool first = d < f.best || f.id == kInvalid;
+            doubt = (first ? false : doubt) || !(nd <= d);
+            if (first || info > rank)
+            {
+                f = Found2{d, child - ni};
+                rank = info;
+                lim = reach2(used, sqrtf(d));
+            }
+        }
+        const bool pL = ok[0] && ch.x < ni && !(md[0] > lim), pR = ok[1] && ch.y < ni && !(md[1] > lim);
+        if (pL || pR)
+        {
+            const bool left = pL && (!pR || md[0] <= md[1]);
+            if (pL && pR)
+            {
+                if (sp >= kStackDepth)
+                {
+                    doubt = true;
+                    break;
+                }
+                sn[sp] = left ? ch.y : ch.x;
+                sd[sp++] = left ? md[1] : md[0];
+            }
+            node = left ? ch.x : ch.y;
+            nd = left ? md[0] : md[1];
+            continue;
+        }
+        while (sp > 0 && sd[sp - 1] > lim)
+            --sp;
+        if (sp == 0)
+            break;
+        --sp;
+        node = sn[sp];
+        nd = sd[sp];
+    }
+    return doubt ? nearest2_in_order(t, p) : f;
 }
 // what a nearest query of this point takes of the margin; unsettled from the start if the
 // coordinates, or the distance to the scene, take all of it (or for a NaN point)
@@ -741,7 +822,7 @@ __global__ void __launch_bounds__(128) nearest2_kernel(Tree2 t, const float *__r
     }
     if (t.n > 1 && (used == INFINITY || (best_pos != kInvalid && !settled2(used, sqrtf(best)))))
     {
-        const Found2 f = nearest2_in_order(t, p);
+        const Found2 f = nearest2_unsettled(t, p);
         best = f.best;
         best_pos = f.id;
     }
@@ -930,6 +1011,82 @@ __device__ __noinline__ Found2 silhouette2_in_order(Tree2 t, float2 p, bool flip
     }
     return f;
 }
+// as nearest2_unsettled
+__device__ __noinline__ Found2 silhouette2_unsettled(Tree2 t, float2 p, bool flip)
+{
+    const uint32_t ni = t.n - 1;
+    const float4 root = __ldg(t.aabbs);
+    const float used = coordinate_ulps(root, p, kSilhouetteUlps);
+    uint32_t sn[kStackDepth];
+    float sd[kStackDepth];
+    Found2 f{INFINITY, (uint32_t)-1};
+    uint32_t key = 0, node = 0;
+    float nd = mindist2(unpack_b2(root), p), lim = INFINITY;
+    bool doubt = false;
+    int sp = 0;
+    for (;;)
+    {
+        const Inner2 *rec = t.inner + node;
+        const Cones2 *cr = t.inner_cones + node;
+        const B2 box[2] = {unpack_b2(__ldg(&rec->lb)), unpack_b2(__ldg(&rec->rb))};
+        const C2 cone[2] = {unpack_c2(__ldg(&cr->l)), unpack_c2(__ldg(&cr->r))};
+        const uint4 ch = __ldg(&rec->ch);
+        float md[2];
+        bool ok[2];
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+        {
+            md[k] = mindist2(box[k], p);
+            ok[k] = !(md[k] > lim) && cone[k].half_angle >= 0.0f && cone_test2(cone[k], p, box[k], md[k]);
+            const uint32_t child = k ? ch.y : ch.x, info = k ? ch.w : ch.z;
+            for (uint32_t e = 0; ok[k] && child >= ni && e < info >> 30; ++e)
+            {
+                const Vert2 *r = t.leaf_verts + 2 * (uint64_t)(child - ni) + e;
+                const float4 va = __ldg(&r->a), vb = __ldg(&r->b);
+                const float2 vd = f2(p.x - va.x, p.y - va.y);
+                const float d = len2(vd);
+                if (!(d <= f.best) || (__float_as_uint(vb.z) == 3u &&
+                                       !is_silhouette_vertex(f2(va.z, va.w), f2(vb.x, vb.y), vd, d, flip)))
+                    continue;
+                const bool first = d < f.best || f.id == (uint32_t)-1;
+                const uint32_t ek = (info & kLeafRankMask) * 4u + e;
+                doubt = (first ? false : doubt) || !(nd <= d * d);
+                if (first || (d > 0.0f ? ek > key : ek < key))
+                {
+                    f = Found2{d, __float_as_uint(vb.w)};
+                    key = ek;
+                    lim = reach2(used, d);
+                }
+            }
+        }
+        const bool pL = ok[0] && ch.x < ni && !(md[0] > lim), pR = ok[1] && ch.y < ni && !(md[1] > lim);
+        if (pL || pR)
+        {
+            const bool left = pL && (!pR || md[0] <= md[1]);
+            if (pL && pR)
+            {
+                if (sp >= kStackDepth)
+                {
+                    doubt = true;
+                    break;
+                }
+                sn[sp] = left ? ch.y : ch.x;
+                sd[sp++] = left ? md[1] : md[0];
+            }
+            node = left ? ch.x : ch.y;
+            nd = left ? md[0] : md[1];
+            continue;
+        }
+        while (sp > 0 && sd[sp - 1] > lim)
+            --sp;
+        if (sp == 0)
+            break;
+        --sp;
+        node = sn[sp];
+        nd = sd[sp];
+    }
+    return doubt ? silhouette2_in_order(t, p, flip) : f;
+}
 SNCH_DEV float silhouette2_ulps(const Tree2 &t, float2 p)  // as nearest2_ulps
 {
     const float4 b = __ldg(t.aabbs);
@@ -1110,8 +1267,8 @@ SNCH_DEV bool nearest2_coop(const Tree2 &t, float2 p, float &best, uint32_t &bes
     }
     return true;
 }
-// The first lane_blocks blocks: a lane per query, for those that replay the reference's
-// order, which gains nothing from a warp.
+// The first lane_blocks blocks: a lane per query, for those that are unsettled from the start
+// (a warp gains nothing on the reference's order).
 __global__ void __launch_bounds__(32 * kCoopWarps, 16)
     nearest2_coop_kernel(Tree2 t, const float *__restrict__ pts, int64_t n, uint32_t *__restrict__ out_idx,
                          float *__restrict__ out_dist, unsigned lane_blocks)
@@ -1125,7 +1282,7 @@ __global__ void __launch_bounds__(32 * kCoopWarps, 16)
         const float2 p = load_pt2(pts, q);
         if (nearest2_ulps(t, p) < INFINITY)
             return;
-        const Found2 f = nearest2_in_order(t, p);
+        const Found2 f = nearest2_unsettled(t, p);
         store_nearest2(t, q, f.best, f.id, out_idx, out_dist);
         return;
     }
@@ -1150,7 +1307,7 @@ __global__ void __launch_bounds__(32 * kCoopWarps, 16)
         return;
     if (best_pos != kInvalid && !settled2(used, sqrtf(best)))
     {
-        const Found2 f = nearest2_in_order(t, p);
+        const Found2 f = nearest2_unsettled(t, p);
         best = f.best;
         best_pos = f.id;
     }
@@ -1250,10 +1407,10 @@ SNCH_DEV void silhouette2_coop_query(const Tree2 &t, const float *__restrict__ p
     {
         const float used = silhouette2_ulps(t, p);
         if (used == INFINITY)
-            return;  // replayed by a lane of its own
+            return;  // answered by a lane of its own
         if (best_vert >= 0 && !settled2(used, best))
         {
-            const Found2 f = silhouette2_in_order(t, p, flip);
+            const Found2 f = silhouette2_unsettled(t, p, flip);
             best = f.best;
             best_vert = (int32_t)f.id;
         }
@@ -1275,7 +1432,7 @@ __global__ void __launch_bounds__(32 * kCoopWarps, 16)
         const float2 p = load_pt2(pts, q);
         if (silhouette2_ulps(t, p) < INFINITY)
             return;
-        const Found2 f = silhouette2_in_order(t, p, flips ? __ldg(flips + q) != 0 : false);
+        const Found2 f = silhouette2_unsettled(t, p, flips ? __ldg(flips + q) != 0 : false);
         out_dist[q] = f.best;
         if (out_vid)
             out_vid[q] = (int32_t)f.id;
@@ -1312,7 +1469,7 @@ __global__ void __launch_bounds__(128) silhouette2_settle_kernel(Tree2 t, const 
     const float d = out_dist[q];  // infinite: none found, so nothing was pruned
     if (settled2(coordinate_ulps(__ldg(t.aabbs), p, kSilhouetteUlps), d < INFINITY ? d : 0.0f))
         return;
-    const Found2 f = silhouette2_in_order(t, p, flips ? __ldg(flips + q) != 0 : false);
+    const Found2 f = silhouette2_unsettled(t, p, flips ? __ldg(flips + q) != 0 : false);
     out_dist[q] = f.best;
     if (out_vid)
         out_vid[q] = (int32_t)f.id;

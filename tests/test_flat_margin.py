@@ -76,3 +76,28 @@ def test_boxes_stay_nearer_inside_the_bound(seed):
     far = np.float64(NEAREST) * top + DISTANCE * d > 40 * LIMIT
     if far.any():
         assert (md[far] > (d * d)[far]).any()
+
+
+@pytest.mark.parametrize("seed", range(4))
+def test_reach_at_every_scale(seed):
+    """What lies beyond reach2 of a distance cannot hold an element at that distance, at any
+    coordinates; and a box that contains another is never farther."""
+    rng = np.random.default_rng(100 + seed)
+    a, b, p = cases(rng, 1_000_000)
+    big = rounded(10 ** rng.uniform(0, 4, len(a)))[:, None]
+    a, b, p = a * big, b * big, p * big
+    top = np.abs(np.concatenate([a, b, p], 1)).max(1) + F(1e-3)
+    md = mindist(a, b, p)
+
+    def reach(d, per_unit):
+        r = d + (per_unit * top + DISTANCE * d) * F(2.0**-24)
+        return r * r * F(1.0000019073486328125)
+
+    d = np.sqrt(segment_sq(a, b, p))
+    assert np.all(md <= reach(np.sqrt(d * d), NEAREST))
+    e = p - a
+    dv = np.sqrt(dot(e, e))
+    assert np.all(md <= reach(dv, SILHOUETTE))
+    c = rounded(a + rng.standard_normal(a.shape) * 10 ** rng.uniform(-4, 4, (len(a), 1)))
+    lo, hi = np.minimum(np.minimum(a, b), c), np.maximum(np.maximum(a, b), c)
+    assert np.all(mindist(lo, hi, p) <= md)
