@@ -246,7 +246,7 @@ SNCH_DEV bool silhouette_coop(const TreeView &t, f3 p, bool flip, uint32_t root,
             }
             __syncwarp();
             for (uint32_t i = lane; i < edges; i += 32)
-                edge_record_candidate(t, items.slot[i], items.key[i], p, flip, cb, ck, ce);
+                edge_record_candidate<true>(t, items.slot[i], items.key[i], p, flip, cb, ck, ce);
             __syncwarp();  // the next step's items overwrite these
         }
         // the best of the lanes' new candidates: smallest distance, then the larger

@@ -775,7 +775,8 @@ SNCH_DEV void leaf_silhouette_fast(const TreeView &t, uint32_t pos, f3 o, bool f
 }
 
 // the edge record at slot (3 x sorted leaf position + edge number) with tie key
-// rank * 4 + edge number, as a silhouette candidate
+// rank * 4 + edge number, as a silhouette candidate; kWide: the normals in one load
+template <bool kWide = false>
 SNCH_DEV void edge_record_candidate(const TreeView &t, uint64_t slot, uint32_t key, f3 o, bool flip, float &best,
                                     uint32_t &best_key, int32_t &best_edge)
 {
@@ -794,9 +795,16 @@ SNCH_DEV void edge_record_candidate(const TreeView &t, uint64_t slot, uint32_t k
     bool is_sil = (flags & 1u) == 0u || (flags & 2u) == 0u;
     if (!is_sil)
     {
-        // two loads: as one of 32 bytes its eight registers in a row made the per-lane search
-        // spill (20,000 queries of a 5,120-triangle sphere 1.79 -> 1.88 ms)
-        const float4 ec = __ldg(e + 2), ed = __ldg(e + 3);
+        // one load of 32 bytes takes eight registers in a row, for which the per-lane search
+        // spills (20,000 queries of a 5,120-triangle sphere 1.79 -> 1.88 ms)
+        float4 ec, ed;
+        if (kWide)
+            load32(e + 2, ec, ed);
+        else
+        {
+            ec = __ldg(e + 2);
+            ed = __ldg(e + 3);
+        }
         is_sil = is_silhouette_edge(pa, pb, mk(ec.x, ec.y, ec.z), mk(ed.x, ed.y, ed.z),
                                     mk(o.x - cp.x, o.y - cp.y, o.z - cp.z), d, flip);
     }
